@@ -571,40 +571,57 @@ cudaError_t zsymtri_prep(const double* ev, const double* dvim, int n, double* dg
   return cudaGetLastError();
 }
 
-// number of eigenvalues of S smaller than x (pivots of LDL^T(S - x I), pivmin guard)
-__device__ int zsturm(const double* dg, const double* off, int n, double x, double pivmin) {
-  double q = dg[0] - x;
-  if (fabs(q) <= pivmin) q = neg(pivmin);
-  int c = (q < 0.0);
-  for (int i = 1; i < n; i++) {
-    const double e = off[i - 1];
-    q = (dg[i] - x) - (e * e) / q;
-    if (fabs(q) <= pivmin) q = neg(pivmin);
-    c += (q < 0.0);
-  }
-  return c;
-}
-
 // mu_k = k-th smallest eigenvalue of S by a group of p lanes (multisection,
-// absolute tolerance eps * max|Gershgorin bound|); vals_im[k] = -mu_k
-__global__ void zbisect_kernel(const double* __restrict__ dg, const double* __restrict__ off, int n, int batch,
+// absolute tolerance eps * max|Gershgorin bound|); vals_im[k] = -mu_k.  Problem
+// blockIdx.y; the scaled diagonal and squares are staged for the CTA up to
+// n = STURM_STAGE.
+__global__ void zbisect_kernel(const double* __restrict__ dg, const double* __restrict__ off, int n,
                                const double* __restrict__ bp, double* __restrict__ mu, double* __restrict__ vals_im,
                                int p) {
-  const long long gid = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / p;
+  extern __shared__ double sq[];
+  const int k0 = (blockIdx.x * blockDim.x + threadIdx.x) / p;
   const int gl = (threadIdx.x & 31) % p;
-  const bool active = gid < (long long)n * batch;
-  const size_t mb = active ? (size_t)(gid / n) : 0;
-  const int k = active ? (int)(gid - (long long)mb * n) : 0;
+  const bool active = k0 < n;
+  const int k = active ? k0 : 0;
+  const size_t mb = blockIdx.y;
   dg += mb * n;
   off += mb * n;
   bp += mb * 8;
-  const double lo = bp[0], hi = bp[2], pivmin = bp[1];
-  const double x = group_multisect(lo, hi, active ? k : 0, 2.220446049250313e-16 * fmax(fabs(lo), fabs(hi)), p,
-                                   active, [&](double y) { return zsturm(dg, off, n, y, pivmin); });
+  const double lo = bp[0], hi = bp[2], scale = sturm_scale(fmax(fabs(lo), fabs(hi)));
+  double* sd = sq + n;
+  const bool staged = n <= STURM_STAGE;
+  if (staged) {
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+      const double v = (i + 1 < n) ? off[i] * scale : 0.0;
+      sq[i] = v * v;
+      sd[i] = dg[i] * scale;
+    }
+    __syncthreads();
+  }
+  auto count = [&](double y) {
+    const double x = y * scale;
+    if (staged) return sturm_products(n, [&](int i) { return sd[i] - x; }, [&](int i) { return sq[i]; });
+    return sturm_products(n, [&](int i) { return fma(dg[i], scale, neg(x)); }, [&](int i) {
+      const double v = off[i] * scale;
+      return v * v;
+    });
+  };
+  const double x = group_multisect(lo, hi, k, 2.220446049250313e-16 * fmax(fabs(lo), fabs(hi)), p, active, count);
   if (active && gl == 0) {
     if (mu) mu[mb * n + k] = x;
     vals_im[mb * n + k] = neg(x);
   }
+}
+
+static cudaError_t launch_zbisect(const double* dg, const double* off, int n, int batch, const double* bp, double* mu,
+                                  double* vals_im, cudaStream_t st) {
+  int dev = 0, sms = 148;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int p = multisect_lanes(n * batch, sms);
+  const unsigned ctas = (unsigned)(((long long)n * p + 127) / 128);
+  const size_t smem = n <= STURM_STAGE ? 2 * n * sizeof(double) : 0;
+  zbisect_kernel<<<dim3(ctas, batch), 128, smem, st>>>(dg, off, n, bp, mu, vals_im, p);
+  return cudaGetLastError();
 }
 
 // V(:, k) = D Y(:, k)
@@ -797,12 +814,7 @@ cudaError_t zeigen_from_tridiag(const double* Ad, int64_t lda, int n, const doub
   zc* Tg = reinterpret_cast<zc*>(Y + seg(B * n * n));
   double* tws = Y + seg(B * n * n) + seg(2 * B * std::max(npan, 1) * ZWB * ZWB);
   zprep_kernel<<<batch, 1024, 0, st>>>(ev, dvim, n, dg, off, ph, bp);
-  int dev = 0, sms = 148;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int p = multisect_lanes(n * batch, sms);
-  const long long threads = ((long long)n * batch * p + 31) / 32 * 32;
-  zbisect_kernel<<<(unsigned)((threads + 127) / 128), 128, 0, st>>>(dg, off, n, batch, bp, mu, vals_im, p);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = launch_zbisect(dg, off, n, batch, bp, mu, vals_im, st);
   if (e != cudaSuccess || !Vd) return e;
   e = symtri_vectors(dg, off, n, mu, bp, Y, tws, batch, st);
   if (e != cudaSuccess) return e;
@@ -965,12 +977,7 @@ cudaError_t zeigen_tridiag(const double* evd, const double* dvim, int n, double*
   const int npan = (n - 1 + ZWB - 1) / ZWB;
   double* tws = Y + seg((size_t)n * n) + seg(2 * (size_t)std::max(npan, 1) * ZWB * ZWB);
   zprep_tri_kernel<<<1, 1024, 0, st>>>(reinterpret_cast<const zc*>(evd), dvim, n, dg, off, ph, bp);
-  int dev = 0, sms = 148;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int p = multisect_lanes(n, sms);
-  const long long threads = ((long long)n * p + 31) / 32 * 32;
-  zbisect_kernel<<<(unsigned)((threads + 127) / 128), 128, 0, st>>>(dg, off, n, 1, bp, mu, vals_im, p);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = launch_zbisect(dg, off, n, 1, bp, mu, vals_im, st);
   if (e != cudaSuccess || !Vd) return e;
   e = symtri_vectors(dg, off, n, mu, bp, Y, tws, 1, st);
   if (e != cudaSuccess) return e;

@@ -297,6 +297,26 @@ __global__ void bisect_prep_kernel(const double* __restrict__ e, int n, double* 
   }
 }
 
+// Squares of the scaled off-diagonal, staged for the CTA (n <= STURM_STAGE), and the
+// Sturm count of SymTridiagonal(0, e) at x from them or from e itself.
+__device__ __forceinline__ void stage_squares(const double* __restrict__ e, int n, double scale, double* sq) {
+  if (n > STURM_STAGE) return;
+  for (int i = threadIdx.x; i + 1 < n; i += blockDim.x) {
+    const double v = e[i] * scale;
+    sq[i] = v * v;
+  }
+  __syncthreads();
+}
+__device__ __forceinline__ int sturm_zero_diag(const double* __restrict__ e, int n, double scale, const double* sq,
+                                               double x) {
+  const double nx = neg(x * scale);
+  if (n <= STURM_STAGE) return sturm_products(n, [&](int) { return nx; }, [&](int i) { return sq[i]; });
+  return sturm_products(n, [&](int) { return nx; }, [&](int i) {
+    const double v = e[i] * scale;
+    return v * v;
+  });
+}
+
 // The positive eigenvalues of SymTridiagonal(0, e): the k-th largest (k < n/2) by
 // a group of p lanes (multisection to relative precision: the zero-diagonal Sturm
 // count resolves the tiny singular values of the bidiagonal coupling, and their
@@ -304,14 +324,16 @@ __global__ void bisect_prep_kernel(const double* __restrict__ e, int n, double* 
 // written together; odd n: vals[n/2] = 0.
 __global__ void bisect_kernel_dev(const double* __restrict__ e, int n, const double* __restrict__ bp,
                                   double* __restrict__ vals, int p) {
+  extern __shared__ double sq[];
   const int h = n / 2;
   const int gid = (blockIdx.x * blockDim.x + threadIdx.x) / p;  // eigenvalue index of the lane's group
   const int gl = (threadIdx.x & 31) % p;
   if ((n & 1) && gid == 0 && gl == 0 && blockIdx.x == 0) vals[h] = 0.0;
-  const double bound = bp[0], pivmin = bp[1];
+  const double bound = bp[0], pivmin = bp[1], scale = sturm_scale(bound);
+  stage_squares(e, n, scale, sq);
   const bool active = gid < h;
   const double x = group_multisect(0.0, bound, n - 1 - (active ? gid : 0), 4.0 * pivmin, p, active,
-                                   [&](double y) { return sturm_count(e, n, y, pivmin); });
+                                   [&](double y) { return sturm_zero_diag(e, n, scale, sq, y); });
   if (active && gl == 0) {
     vals[gid] = x;
     vals[n - 1 - gid] = neg(x);
@@ -327,7 +349,8 @@ cudaError_t launch_tridiag_bisect(const double* ev, int n, double* vals_im, doub
   const int p = multisect_lanes(h, sms);
   const long long threads = ((long long)std::max(h, 1) * p + 31) / 32 * 32;
   const int bs = 128;
-  bisect_kernel_dev<<<(unsigned)((threads + bs - 1) / bs), bs, 0, st>>>(ev, n, scratch2, vals_im, p);
+  const size_t smem = n <= STURM_STAGE ? n * sizeof(double) : 0;
+  bisect_kernel_dev<<<(unsigned)((threads + bs - 1) / bs), bs, smem, st>>>(ev, n, scratch2, vals_im, p);
   return cudaGetLastError();
 }
 
@@ -367,6 +390,7 @@ __global__ void bisect_prep_batch_kernel(const double* __restrict__ e_g, int n, 
 __global__ void bisect_batch_kernel(const double* __restrict__ e_g, int n, const double* __restrict__ bp_g,
                                     double* __restrict__ vals_g, double* const* __restrict__ vals_out,
                                     const int32_t* __restrict__ idx, int p) {
+  extern __shared__ double sq[];
   const int mb = blockIdx.y;
   const double* e = e_g + (size_t)mb * n;
   const double* bp = bp_g + (size_t)mb * 8;
@@ -379,10 +403,11 @@ __global__ void bisect_batch_kernel(const double* __restrict__ e_g, int n, const
     vals[h] = 0.0;
     out[h] = 0.0;
   }
-  const double bound = bp[0], pivmin = bp[1];
+  const double bound = bp[0], pivmin = bp[1], scale = sturm_scale(bound);
+  stage_squares(e, n, scale, sq);
   const bool active = gid < h;
   const double x = group_multisect(0.0, bound, n - 1 - (active ? gid : 0), 4.0 * pivmin, p, active,
-                                   [&](double y) { return sturm_count(e, n, y, pivmin); });
+                                   [&](double y) { return sturm_zero_diag(e, n, scale, sq, y); });
   if (active && gl == 0) {
     vals[gid] = x;
     vals[n - 1 - gid] = neg(x);
@@ -404,8 +429,9 @@ cudaError_t launch_tridiag_bisect_batch(const double* e_g, int n, int G, double*
   const int p = multisect_lanes(std::max(1, h * G), sms);
   const long long threads = ((long long)std::max(h, 1) * p + 31) / 32 * 32;
   const int bs = 128;
-  bisect_batch_kernel<<<dim3((unsigned)((threads + bs - 1) / bs), G), bs, 0, st>>>(e_g, n, bp_g, vals_g, vals_out,
-                                                                                   idx, p);
+  const size_t smem = n <= STURM_STAGE ? n * sizeof(double) : 0;
+  bisect_batch_kernel<<<dim3((unsigned)((threads + bs - 1) / bs), G), bs, smem, st>>>(e_g, n, bp_g, vals_g, vals_out,
+                                                                                      idx, p);
   return cudaGetLastError();
 }
 
