@@ -83,6 +83,7 @@ struct skew_batch_plan_st {
   double** e_p_work = nullptr;     // work + off_w per matrix
   int* e_status = nullptr;
   unsigned* e_counter = nullptr;
+  int* e_exps = nullptr;  // exponents of the tiled products' operands (2 x ev_total)
   int* e_fsel = nullptr;  // exp adjoint: per matrix, real Schur-basis (1) or complex (0) form
   int32_t* e_back_off = nullptr;  // back-transformation items before each matrix (processing order)
   int32_t back_items = 0;
@@ -637,7 +638,7 @@ int skew_batch_plan_destroy(skew_batch_plan_t P) {
   if (P->d_gws) cudaFreeAsync(P->d_gws, st);
   void* eig[] = {P->e_refl, P->e_tau, P->e_evb, P->e_G, P->e_log, P->e_work, P->e_vr, P->e_vi, P->e_vals,
                  P->e_off_log, P->e_cap_log, P->e_log_len, P->e_off_w, P->e_p_refl, P->e_p_vr, P->e_p_vi,
-                 P->e_p_vals, P->e_p_scratch, P->e_p_work, P->e_status, P->e_fsel, P->e_back_off,
+                 P->e_p_vals, P->e_p_scratch, P->e_p_work, P->e_status, P->e_fsel, P->e_exps, P->e_back_off,
                  P->e_counter};
   for (void* q : eig)
     if (q) cudaFreeAsync(q, st);
@@ -934,6 +935,7 @@ static int eigen_ws(skew_batch_plan_t P) {
   alloc((void**)&P->e_p_work, sizeof(double*) * count);
   alloc((void**)&P->e_status, sizeof(int) * count);
   alloc((void**)&P->e_fsel, sizeof(int) * count);
+  alloc((void**)&P->e_exps, sizeof(int) * 2 * P->ev_total);
   alloc((void**)&P->e_back_off, sizeof(int32_t) * (count + 1));
   alloc((void**)&P->e_counter, sizeof(unsigned));
   if (!ok) return SKEW_NO_MEMORY;
@@ -1089,6 +1091,8 @@ static int eigen_run(skew_batch_plan_t P, const double* const* A, double* const*
   E.out = nullptr;
   E.cot = nullptr;
   E.pwork = P->e_p_work;
+  E.exps = P->e_exps;
+  E.exps_stride = P->ev_total;
   E.func = SKEW_FUNC_EXP;
   E.merged = ev_in ? 1 : 0;
   E.chain_nmax = (ev_in || chain_nmax >= P->nmax) ? (1 << 30) : chain_nmax;
@@ -1284,13 +1288,13 @@ static int eigen_large(skew_handle_t h, double* A, int64_t n, int64_t lda, doubl
 // bisection and twisted vectors of the tridiagonal ev; then the element-wise step
 // and the tiled products of the batched path run on them as a batch of one.  The
 // eigenvalue order (descending here) does not change these functions.
-// Handle aux layout (doubles): [Vr n^2][Vi n^2][work 4 n^2][vals n][8 pointers][n, status].
+// Handle aux layout (doubles): [Vr n^2][Vi n^2][work 4 n^2][vals n][8 pointers][n, status][exponents n].
 static int func_large(skew_handle_t h, double* A, const double* ev, int64_t n, double* out, const double* cot,
                       int mode, int func, int* info) {
   if (!h || !out || (mode == 2 && !cot)) return SKEW_BAD_ARG;
   if (n > (1LL << 15)) return SKEW_UNSUPPORTED;
   const size_t nn = (size_t)n * (size_t)n;
-  int st = ensure_aux(h, sizeof(double) * (6 * nn + (size_t)n + 8 + 2));
+  int st = ensure_aux(h, sizeof(double) * (6 * nn + 2 * (size_t)n + 8 + 2));
   if (st) return st;
   cudaStream_t s = h->stream;
   double* Vr = (double*)h->aux;
@@ -1300,6 +1304,7 @@ static int func_large(skew_handle_t h, double* A, const double* ev, int64_t n, d
   double** ptrs = (double**)(vals + n);  // [0] Vr, [1] Vi, [2] vals, [3] work, [4] out, [5] cot
   int32_t* dn = (int32_t*)(ptrs + 8);
   int* status = (int*)(dn + 1);
+  int* exps = (int*)(ptrs + 8 + 2);
   const int32_t n32 = (int32_t)n;
   CK(cudaMemcpyAsync(dn, &n32, sizeof(int32_t), cudaMemcpyHostToDevice, s));  // pageable: staged before return
   CK(cudaMemsetAsync(status, 0, sizeof(int), s));
@@ -1320,6 +1325,8 @@ static int func_large(skew_handle_t h, double* A, const double* ev, int64_t n, d
   E.Vr = ptrs;
   E.Vi = ptrs + 1;
   E.pwork = ptrs + 3;
+  E.exps = exps;
+  E.exps_stride = n;
   E.out = ptrs + 4;
   E.cot = (const double* const*)(ptrs + 5);
   E.func = func;

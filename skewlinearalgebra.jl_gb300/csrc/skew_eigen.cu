@@ -37,6 +37,7 @@
 #include "skew_internal.h"
 #include "skew_twisted.cuh"
 #include "skew_funcs.cuh"
+#include "skew_oz.cuh"
 
 namespace skew {
 
@@ -683,96 +684,155 @@ struct BOperand {
 
 struct BGemm {
   const int32_t* n;
-  const int* status;  // matrices with SKEW_NO_CONVERGENCE are skipped
+  int* status;        // matrices with SKEW_NO_CONVERGENCE are skipped
   const int* sel;     // non-null: only matrices with sel[b] == sel_val
   int sel_val;
-  int nterms;         // C_b = sum_t s_t op(A_t,b) op(B_t,b)
+  int nterms;         // C_b = sum_t s_t op(A_t,b) op(B_t,b), s_t = +-1, both terms transposed alike
   BOperand A[2], B[2];
   double s[2];
   double* const* C;
   int c_add_sq;
   int c_add;   // extra offset in doubles (1: imaginary parts of an interleaved output)
   int c_step;  // 1, or 2 for a ComplexF64 output
+  const int64_t* off_n;  // packed vector offset per matrix (null: one matrix)
+  int* exps;             // [2 nterms][exps_stride]: largest exponents of op(A)'s rows, op(B)'s columns
+  int64_t exps_stride;
 };
 
-constexpr int BG_T = 64, BG_K = 16;
-
-// One 64 x 64 tile of one matrix per CTA: grid (tiles^2 of the largest matrix, count);
-// tiles outside a smaller matrix return at once.
-__global__ void __launch_bounds__(256) bgemm_kernel(BGemm P) {
-  __shared__ double As[BG_K][BG_T + 1];
-  __shared__ double Bs[BG_K][BG_T + 1];
+// Largest exponents of the rows of op(A) and the columns of op(B) over all terms: grid
+// (blocks of 64 vectors of the largest matrix, count, 2), z = 0: A, 1: B.
+__global__ void __launch_bounds__(256) bgemm_exps_kernel(BGemm P) {
+  __shared__ int red[4][64];
   const int b = blockIdx.y;
   const int n = P.n[b];
   if (P.status && P.status[b] == SKEW_NO_CONVERGENCE) return;
   if (P.sel && P.sel[b] != P.sel_val) return;
-  const int nt = (n + BG_T - 1) / BG_T;
-  if ((int)blockIdx.x >= nt * nt) return;
-  const int i0 = (blockIdx.x % nt) * BG_T, j0 = (blockIdx.x / nt) * BG_T;
-  const int64_t nn = (int64_t)n * n;
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  double acc[4][4];
+  const int i0 = blockIdx.x * 64;
+  if (i0 >= n) return;
+  const int side = blockIdx.z;
+  int* ex = P.exps + side * P.exps_stride + (P.off_n ? P.off_n[b] : 0);
+  int e[8];  // across the columns: e[0] of vector tid % 64; along: of vectors tid / 32 + 8 q
 #pragma unroll
-  for (int a = 0; a < 4; a++)
-#pragma unroll
-    for (int q = 0; q < 4; q++) acc[a][q] = 0.0;
+  for (int q = 0; q < 8; q++) e[q] = 1;
   for (int t = 0; t < P.nterms; t++) {
-    const double* A = P.A[t].p[b] + (int64_t)P.A[t].add_sq * nn;
-    const double* B = P.B[t].p[b] + (int64_t)P.B[t].add_sq * nn;
-    const int ta = P.A[t].trans, tb = P.B[t].trans;
-    const double sg = P.s[t];
-    for (int k0 = 0; k0 < n; k0 += BG_K) {
+    const BOperand& O = side ? P.B[t] : P.A[t];
+    const double* M = O.p[b] + (int64_t)O.add_sq * n * n;
+    if ((O.trans != 0) == (side != 0)) {  // the vectors lie across the columns of M
+      const int ii = threadIdx.x & 63, kg = threadIdx.x >> 6;
+      int m = 1;
+      if (i0 + ii < n)
+        for (int k = kg; k < n; k += 4) m = max(m, oz_exponent(M[i0 + ii + (int64_t)k * n]));
       __syncthreads();
-      for (int idx = threadIdx.x; idx < BG_T * BG_K; idx += 256) {
-        int ii, kk;
-        if (!ta) {
-          ii = idx & 63;
-          kk = idx >> 6;
-        } else {
-          kk = idx & 15;
-          ii = idx >> 4;
-        }
-        const int i = i0 + ii, k = k0 + kk;
-        double av = 0.0;
-        if (i < n && k < n) av = ta ? A[k + (int64_t)i * n] : A[i + (int64_t)k * n];
-        As[kk][ii] = sg * av;
-        int jj, kb;
-        if (!tb) {
-          kb = idx & 15;
-          jj = idx >> 4;
-        } else {
-          jj = idx & 63;
-          kb = idx >> 6;
-        }
-        const int j = j0 + jj, k2 = k0 + kb;
-        double bv = 0.0;
-        if (j < n && k2 < n) bv = tb ? B[j + (int64_t)k2 * n] : B[k2 + (int64_t)j * n];
-        Bs[kb][jj] = bv;
+      red[kg][ii] = m;
+      __syncthreads();
+      const int ia = threadIdx.x >> 5;
+#pragma unroll
+      for (int q = 0; q < 8; q++) {
+        const int i = ia + 8 * q;
+        e[q] = max(e[q], max(max(red[0][i], red[1][i]), max(red[2][i], red[3][i])));
       }
-      __syncthreads();
+    } else {  // each vector is a column of M
 #pragma unroll
-      for (int kk = 0; kk < BG_K; kk++) {
-        double a4[4], b4[4];
-#pragma unroll
-        for (int a = 0; a < 4; a++) {
-          a4[a] = As[kk][tx + 16 * a];
-          b4[a] = Bs[kk][ty + 16 * a];
-        }
-#pragma unroll
-        for (int a = 0; a < 4; a++)
-#pragma unroll
-          for (int q = 0; q < 4; q++) acc[a][q] = fma(a4[a], b4[q], acc[a][q]);
+      for (int q = 0; q < 8; q++) {
+        const int i = i0 + (threadIdx.x >> 5) + 8 * q;
+        int m = 1;
+        if (i < n)
+          for (int k = threadIdx.x & 31; k < n; k += 32) m = max(m, oz_exponent(M[k + (int64_t)i * n]));
+        e[q] = max(e[q], __reduce_max_sync(0xffffffffu, m));
       }
     }
   }
-  double* C = P.C[b] + (int64_t)P.c_add_sq * nn + P.c_add;
+  if ((threadIdx.x & 31) == 0) {
 #pragma unroll
-  for (int a = 0; a < 4; a++)
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-      const int i = i0 + tx + 16 * a, j = j0 + ty + 16 * q;
-      if (i < n && j < n) C[(int64_t)P.c_step * (i + (int64_t)j * n)] = acc[a][q];
+    for (int q = 0; q < 8; q++) {
+      const int i = i0 + (threadIdx.x >> 5) + 8 * q;
+      if (i < n) ex[i] = e[q];
     }
+  }
+}
+
+// One matrix of the batched product for oz_tile: the terms lie one after the other along
+// K, each padded to whole buffers.
+struct BGemmTile {
+  const double* A[2];
+  const double* B[2];
+  int ta[2], tb[2], neg[2];
+  int n, per, terms;  // buffers of OZ_K per term
+  const int *ea, *eb;
+  double* C;
+  int c_step;
+  int* status;
+  __device__ int rows() const { return n; }
+  __device__ int cols() const { return n; }
+  __device__ int ksteps() const { return per * terms; }
+  __device__ bool contiguousA() const { return ta[0]; }
+  __device__ bool contiguousB() const { return !tb[0]; }
+  __device__ int expA(int i) const { return ea[i]; }
+  __device__ int expB(int j) const { return eb[j]; }
+  // NV entries from k of vector i of M (across: vectors lie across the columns)
+  template <int NV>
+  __device__ __forceinline__ void load(const double* M, bool across, int i, int k, double (&v)[NV]) const {
+    const double* p = across ? M + i + (int64_t)k * n : M + k + (int64_t)i * n;
+    const int64_t st = across ? n : 1;
+    if (k + NV <= n) {
+#pragma unroll
+      for (int u = 0; u < NV; u++) v[u] = p[u * st];
+    } else {
+#pragma unroll
+      for (int u = 0; u < NV; u++) v[u] = (k + u < n) ? p[u * st] : 0.0;
+    }
+  }
+  __device__ void loadA(int i, int s, int k, double (&v)[8]) const {
+    const int t = s >= per;
+    load<8>(A[t], !ta[t], i, (s - t * per) * OZ_K + k, v);
+    if (neg[t]) {
+#pragma unroll
+      for (int u = 0; u < 8; u++) v[u] = skew::neg(v[u]);
+    }
+  }
+  __device__ void loadB(int j, int s, int k, double (&v)[4]) const {
+    const int t = s >= per;
+    load<4>(B[t], tb[t], j, (s - t * per) * OZ_K + k, v);
+  }
+  __device__ void store(int i, int j, double x) const { C[(int64_t)c_step * (i + (int64_t)j * n)] = x; }
+  __device__ void timeout() const {
+    if (status) *status = SKEW_TIMEOUT;
+  }
+};
+
+// One 128 x 64 tile of one matrix per CTA: grid (tiles of the largest matrix, count);
+// tiles outside a smaller matrix return at once.  On the tensor cores (skew_oz.cuh): the
+// products were FP64-pipe bound (1.1 TFLOP/s); now bound by cutting the entries into
+// digits (27 integer instructions each, 64 lanes per clock and SM) next to the MMAs.
+// 2048^3: 14.2 -> 0.76 ms; the four products of the 512-matrix exp adjoint:
+// 147.2 -> 11.5 ms.
+__global__ void __launch_bounds__(OZ_NT, 1) bgemm_kernel(BGemm P) {
+  extern __shared__ __align__(1024) unsigned char oz_buf[];
+  const int b = blockIdx.y;
+  const int n = P.n[b];
+  if (P.status && P.status[b] == SKEW_NO_CONVERGENCE) return;
+  if (P.sel && P.sel[b] != P.sel_val) return;
+  const int mt = (n + OZ_M - 1) / OZ_M, nt = (n + OZ_N - 1) / OZ_N;
+  if ((int)blockIdx.x >= mt * nt) return;
+  const int64_t nn = (int64_t)n * n;
+  BGemmTile T;
+#pragma unroll
+  for (int t = 0; t < 2; t++) {
+    T.A[t] = P.A[t].p[b] + (int64_t)P.A[t].add_sq * nn;
+    T.B[t] = P.B[t].p[b] + (int64_t)P.B[t].add_sq * nn;
+    T.ta[t] = P.A[t].trans;
+    T.tb[t] = P.B[t].trans;
+    T.neg[t] = P.s[t] < 0.0;
+  }
+  T.n = n;
+  T.per = (n + OZ_K - 1) / OZ_K;
+  T.terms = P.nterms;
+  T.ea = P.exps + (P.off_n ? P.off_n[b] : 0);
+  T.eb = T.ea + P.exps_stride;
+  T.C = P.C[b] + (int64_t)P.c_add_sq * nn + P.c_add;
+  T.c_step = P.c_step;
+  T.status = P.status ? P.status + b : nullptr;
+  oz_tile(T, (int)(blockIdx.x % mt) * OZ_M, (int)(blockIdx.x / mt) * OZ_N, oz_buf);
 }
 
 // Elementwise steps, grid (chunks, count):
@@ -867,8 +927,18 @@ static cudaError_t bgemm(const EigenBatch& E, int nterms, BOperand A0, BOperand 
   P.c_add_sq = c_add_sq;
   P.c_add = c_add;
   P.c_step = c_step;
-  const int nt = (E.nmax + BG_T - 1) / BG_T;
-  bgemm_kernel<<<dim3(nt * nt, E.count), 256, 0, st>>>(P);
+  P.off_n = E.off_n;
+  P.exps = E.exps;
+  P.exps_stride = E.exps_stride;
+  P.off_n = E.off_n;
+  P.exps = E.exps;
+  P.exps_stride = E.exps_stride;
+  static std::atomic<uint64_t> raised{0};
+  cudaError_t e = raise_smem_limit_once((const void*)bgemm_kernel, raised);
+  if (e != cudaSuccess) return e;
+  const int tiles = ((E.nmax + OZ_M - 1) / OZ_M) * ((E.nmax + OZ_N - 1) / OZ_N);
+  bgemm_exps_kernel<<<dim3((E.nmax + 63) / 64, E.count, 2), 256, 0, st>>>(P);
+  bgemm_kernel<<<dim3(tiles, E.count), OZ_NT, OZ_SMEM, st>>>(P);
   return cudaGetLastError();
 }
 

@@ -249,6 +249,9 @@ struct EigenBatch {
   double* const* out;        // [count] exp (real) / cis (complex interleaved) / adjoint (real)
   const double* const* cot;  // [count] cotangents for the adjoint
   double* const* pwork;      // [count] work + off_w (pointer array for the tiled products)
+  int* exps = nullptr;       // 2 x exps_stride: largest exponents per operand vector of the tiled products,
+                             // packed like off_n
+  int64_t exps_stride = 0;
   int func;                  // skew_func_t of mode 0 (exp and the other matrix functions)
   int merged;                // 1: skewtrieigen_merged! (tridiagonal input; no mem deflation of :355)
   int chain_nmax;            // matrices with n > chain_nmax skip the QR chain and its vectors
