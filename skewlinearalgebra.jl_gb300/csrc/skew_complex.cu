@@ -26,11 +26,11 @@
 
 #include <algorithm>
 
+#include "skew_internal.h"
+#include "skew_back.cuh"
 #include "skew_common.cuh"
 #include "skew_complex.cuh"
 #include "skew_funcs.cuh"
-#include "skew_internal.h"
-#include "skew_oz.cuh"
 
 namespace skew {
 
@@ -640,161 +640,44 @@ __global__ void zassemble_kernel(const double* __restrict__ Y, const zc* __restr
 }
 
 // ---------------------------------------------------------------------------
-// complex compact WY: Q_b = H_c0 ... H_c1-1 = I - V T V^H, T(i,i) = tau_i,
-// T(0:i, i) = -tau_i T(0:i, 0:i) (V(:, 0:i)^H v_i); X <- Q X by strips
+// X <- Q X (skew_back.cuh): problem b at A + lda n b, tau + n b, X + ldx n b (complex)
 // ---------------------------------------------------------------------------
-constexpr int ZWB = 32;  // reflectors per panel
-constexpr int ZSW = 16;  // complex columns per strip
-constexpr int ZRC = 16;  // rows per staged chunk (one X element per thread)
-
-__device__ __forceinline__ zc zrefl_at(const zc* A, int64_t lda, const zc* tau, int row, int c) {
-  if (row < c + 1 || (tau[c].re == 0.0 && tau[c].im == 0.0)) return zc{0.0, 0.0};
-  return (row == c + 1) ? zc{1.0, 0.0} : A[row + (int64_t)c * lda];
-}
-
-__global__ void __launch_bounds__(256) zwy_factor_kernel(const zc* __restrict__ A, int64_t lda,
-                                                         const zc* __restrict__ tau, int n, zc* __restrict__ Tg) {
-  __shared__ zc Vs[16][ZWB + 1];
-  __shared__ zc M[ZWB][ZWB + 1];  // lower: G = V^H V, upper + diagonal: T
-  const size_t mb = blockIdx.y;   // problem mb: A lda*n, tau n, T gridDim.x panels apart
-  A += mb * (size_t)lda * n;
-  tau += mb * n;
-  Tg += mb * gridDim.x * (size_t)ZWB * ZWB;
-  const int b = blockIdx.x;
-  const int c0 = b * ZWB, c1 = min(c0 + ZWB, n - 1), nb = c1 - c0;
-  const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;  // G (32 x 32): 2 x 2 per thread
-  zc acc[2][2] = {{{0.0, 0.0}, {0.0, 0.0}}, {{0.0, 0.0}, {0.0, 0.0}}};
-  for (int r0 = c0 + 1; r0 < n; r0 += 16) {
-    __syncthreads();
-    for (int idx = threadIdx.x; idx < 16 * ZWB; idx += 256) {
-      const int cc = idx / 16, rr = idx - cc * 16;
-      const int row = r0 + rr;
-      Vs[rr][cc] = (row < n && cc < nb) ? zrefl_at(A, lda, tau, row, c0 + cc) : zc{0.0, 0.0};
-    }
-    __syncthreads();
-    for (int rr = 0; rr < 16; rr++) {
-#pragma unroll
-      for (int a = 0; a < 2; a++)
-#pragma unroll
-        for (int q = 0; q < 2; q++) acc[a][q] = zfma(zconj(Vs[rr][ty + 16 * a]), Vs[rr][tx + 16 * q], acc[a][q]);
-    }
+struct ZBack {
+  BackTask<true> B;  // problem 0
+  size_t stride;     // doubles of workspace per problem
+  __device__ bool get(int b, BackTask<true>& T) const {
+    T = B;
+    T.A += 2 * (size_t)b * B.lda * B.n;
+    T.tau += 2 * (size_t)b * B.n;
+    T.X[0] += 2 * (size_t)b * B.ldx * B.n;
+    const size_t o = b * stride;
+    T.t += o;
+    T.vt += o;
+    T.w += o;
+    T.et += 2 * o;
+    T.evt += 2 * o;
+    T.ex += 2 * o;
+    return true;
   }
-  __syncthreads();
-#pragma unroll
-  for (int a = 0; a < 2; a++)
-#pragma unroll
-    for (int q = 0; q < 2; q++) {
-      const int i = ty + 16 * a, j = tx + 16 * q;  // acc = v_i^H v_j = G(i, j)
-      M[i][j] = (i > j) ? acc[a][q] : zc{0.0, 0.0};
-    }
-  __syncthreads();
-  for (int i = 0; i < nb; i++) {
-    const zc ti = tau[c0 + i];
-    if (threadIdx.x < i) {
-      const int j = threadIdx.x;
-      zc s{0.0, 0.0};
-      for (int l = j; l < i; l++) s = zfma(M[j][l], zconj(M[i][l]), s);  // G(l, i) = conj(G(i, l))
-      M[j][i] = zmul(zc{neg(ti.re), neg(ti.im)}, s);
-    }
-    if (threadIdx.x == 0) M[i][i] = ti;
-    __syncthreads();
-  }
-  zc* T = Tg + (size_t)b * ZWB * ZWB;
-  for (int idx = threadIdx.x; idx < ZWB * ZWB; idx += 256) {
-    const int i = idx / ZWB, j = idx % ZWB;
-    T[idx] = (j >= i) ? M[i][j] : zc{0.0, 0.0};
-  }
-}
-
-__global__ void __launch_bounds__(256) zback_strip_kernel(const zc* __restrict__ A, int64_t lda,
-                                                          const zc* __restrict__ tau, int n, const zc* __restrict__ Tg,
-                                                          int npan, zc* __restrict__ X, int64_t ldx, int ncols) {
-  __shared__ zc Ts[ZWB][ZWB + 1];
-  __shared__ zc Ws[ZWB][ZSW + 1];
-  __shared__ zc Vs[ZRC][ZWB + 1];
-  __shared__ zc Xs[ZRC][ZSW + 1];
-  const size_t mb = blockIdx.y;  // problem mb: A lda*n, tau n, T npan panels, X ldx*ncols apart
-  A += mb * (size_t)lda * n;
-  tau += mb * n;
-  Tg += mb * (size_t)npan * ZWB * ZWB;
-  X += mb * (size_t)ldx * ncols;
-  const int col0 = blockIdx.x * ZSW;
-  const int ncol = min(ZSW, ncols - col0);
-  X += (int64_t)col0 * ldx;
-  // W (32 x 16): 2 per thread (rows wr, wr+16); X chunk (16 x 16): 1 per thread
-  const int wc = threadIdx.x & 15, wr = threadIdx.x >> 4;
-  for (int b = npan - 1; b >= 0; b--) {
-    const int c0 = b * ZWB, c1 = min(c0 + ZWB, n - 1), nb = c1 - c0;
-    __syncthreads();
-    for (int idx = threadIdx.x; idx < ZWB * ZWB; idx += 256) Ts[idx / ZWB][idx % ZWB] = Tg[(size_t)b * ZWB * ZWB + idx];
-    zc w0{0.0, 0.0}, w1{0.0, 0.0};
-    for (int r0 = c0 + 1; r0 < n; r0 += ZRC) {
-      __syncthreads();
-      for (int idx = threadIdx.x; idx < ZRC * ZWB; idx += 256) {
-        const int cc = idx / ZRC, rr = idx - cc * ZRC;
-        const int row = r0 + rr;
-        Vs[rr][cc] = (row < n && cc < nb) ? zrefl_at(A, lda, tau, row, c0 + cc) : zc{0.0, 0.0};
-      }
-      for (int idx = threadIdx.x; idx < ZRC * ZSW; idx += 256) {
-        const int cc = idx / ZRC, rr = idx - cc * ZRC;
-        const int row = r0 + rr;
-        Xs[rr][cc] = (row < n && cc < ncol) ? X[row + (int64_t)cc * ldx] : zc{0.0, 0.0};
-      }
-      __syncthreads();
-#pragma unroll 4
-      for (int rr = 0; rr < ZRC; rr++) {
-        const zc x = Xs[rr][wc];
-        w0 = zfma(zconj(Vs[rr][wr]), x, w0);
-        w1 = zfma(zconj(Vs[rr][wr + 16]), x, w1);
-      }
-    }
-    Ws[wr][wc] = w0;
-    Ws[wr + 16][wc] = w1;
-    __syncthreads();
-    zc t0{0.0, 0.0}, t1{0.0, 0.0};
-    for (int l = wr; l < ZWB; l++) t0 = zfma(Ts[wr][l], Ws[l][wc], t0);
-    for (int l = wr + 16; l < ZWB; l++) t1 = zfma(Ts[wr + 16][l], Ws[l][wc], t1);
-    __syncthreads();
-    Ws[wr][wc] = t0;
-    Ws[wr + 16][wc] = t1;
-    for (int r0 = c0 + 1; r0 < n; r0 += ZRC) {
-      __syncthreads();
-      for (int idx = threadIdx.x; idx < ZRC * ZWB; idx += 256) {
-        const int cc = idx / ZRC, rr = idx - cc * ZRC;
-        const int row = r0 + rr;
-        Vs[rr][cc] = (row < n && cc < nb) ? zrefl_at(A, lda, tau, row, c0 + cc) : zc{0.0, 0.0};
-      }
-      for (int idx = threadIdx.x; idx < ZRC * ZSW; idx += 256) {
-        const int cc = idx / ZRC, rr = idx - cc * ZRC;
-        const int row = r0 + rr;
-        Xs[rr][cc] = (row < n && cc < ncol) ? X[row + (int64_t)cc * ldx] : zc{0.0, 0.0};
-      }
-      __syncthreads();
-      zc a0{0.0, 0.0};
-#pragma unroll 8
-      for (int l = 0; l < ZWB; l++) a0 = zfma(Vs[wr][l], Ws[l][wc], a0);
-      Xs[wr][wc] = zsub(Xs[wr][wc], a0);
-      __syncthreads();
-      for (int idx = threadIdx.x; idx < ZRC * ZSW; idx += 256) {
-        const int cc = idx / ZRC, rr = idx - cc * ZRC;
-        const int row = r0 + rr;
-        if (row < n && cc < ncol) X[row + (int64_t)cc * ldx] = Xs[rr][cc];
-      }
-    }
-  }
-}
+};
 
 // workspace segments are rounded to 32 doubles so that every complex array is 16-byte aligned
 static inline size_t seg(size_t d) { return (d + 31) & ~(size_t)31; }
 
+// The back-transformation's workspace lies in that of the vectors, which are done with it,
+// where it fits (3 n KP doubles per problem; splits of W are chosen to fit).
+static size_t zback_extra_doubles(int n, int batch) {
+  const size_t per = seg(n > 1 ? back_ws_doubles<true>(n, n - 1, n, 1) : 0);
+  return per <= large_eigen_ws_doubles(n) ? 0 : seg((size_t)batch * per);
+}
+
 size_t zeigen_ws_doubles(int n, int batch) {
-  const int npan = (n - 1 + ZWB - 1) / ZWB;
   const size_t B = (size_t)(batch > 0 ? batch : 1);
   return 3 * seg(B * n)                      // dg, off, mu
          + seg(2 * B * n)                    // phases
          + seg(8 * B)                        // bp
          + seg(B * n * n)                    // Y
-         + seg(2 * B * std::max(npan, 1) * ZWB * ZWB)  // T factors
+         + zback_extra_doubles(n, (int)B)
          + B * large_eigen_ws_doubles(n) + 64;
 }
 
@@ -804,7 +687,6 @@ size_t zeigen_ws_doubles(int n, int batch) {
 cudaError_t zeigen_from_tridiag(const double* Ad, int64_t lda, int n, const double* taud, const double* ev,
                                 const double* dvim, double* vals_im, double* Vd, int64_t ldv, double* ws, int batch,
                                 cudaStream_t st) {
-  const int npan = (n - 1 + ZWB - 1) / ZWB;
   const size_t B = (size_t)batch;
   double* dg = ws;
   double* off = dg + seg(B * n);
@@ -812,8 +694,9 @@ cudaError_t zeigen_from_tridiag(const double* Ad, int64_t lda, int n, const doub
   zc* ph = reinterpret_cast<zc*>(mu + seg(B * n));
   double* bp = mu + seg(B * n) + seg(2 * B * n);
   double* Y = bp + seg(8 * B);
-  zc* Tg = reinterpret_cast<zc*>(Y + seg(B * n * n));
-  double* tws = Y + seg(B * n * n) + seg(2 * B * std::max(npan, 1) * ZWB * ZWB);
+  double* extra = Y + seg(B * n * n);
+  const size_t nextra = zback_extra_doubles(n, batch);
+  double* tws = extra + nextra;
   zprep_kernel<<<batch, 1024, 0, st>>>(ev, dvim, n, dg, off, ph, bp);
   cudaError_t e = launch_zbisect(dg, off, n, batch, bp, mu, vals_im, st);
   if (e != cudaSuccess || !Vd) return e;
@@ -823,11 +706,29 @@ cudaError_t zeigen_from_tridiag(const double* Ad, int64_t lda, int n, const doub
   zassemble_kernel<<<dim3((n + 255) / 256, n, batch), 256, 0, st>>>(Y, ph, n, V, ldv);
   e = cudaGetLastError();
   if (e != cudaSuccess || n < 2) return e;
-  const zc* A = reinterpret_cast<const zc*>(Ad);
-  const zc* tau = reinterpret_cast<const zc*>(taud);
-  zwy_factor_kernel<<<dim3(npan, batch), 256, 0, st>>>(A, lda, tau, n, Tg);
-  zback_strip_kernel<<<dim3((n + ZSW - 1) / ZSW, batch), 256, 0, st>>>(A, lda, tau, n, Tg, npan, V, ldv, n);
-  return cudaGetLastError();
+  int dev = 0, sms = 148;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  ZBack S;
+  S.B.A = Ad;
+  S.B.lda = lda;
+  S.B.tau = taud;
+  S.B.n = n;
+  S.B.nref = n - 1;
+  S.B.X[0] = S.B.X[1] = Vd;
+  S.B.ldx = ldv;
+  S.B.nc[0] = n;
+  S.B.nc[1] = 0;
+  S.B.status = nullptr;
+  int splits = 1;
+  if (nextra) {
+    S.stride = seg(back_ws_doubles<true>(n, n - 1, n, 1));
+  } else {
+    S.stride = large_eigen_ws_doubles(n);
+    splits = back_splits(n, batch, sms);
+    while (splits > 1 && back_ws_doubles<true>(n, n - 1, n, splits) > S.stride) splits /= 2;
+  }
+  back_ws_set(S.B, nextra ? extra : tws, n, splits);
+  return back_transform_oz<true>(S, batch, n, n - 1, n, splits, st);
 }
 
 // ---------------------------------------------------------------------------
@@ -1023,8 +924,7 @@ cudaError_t zeigen_tridiag(const double* evd, const double* dvim, int n, double*
   zc* ph = reinterpret_cast<zc*>(mu + seg(n));
   double* bp = mu + seg(n) + seg(2 * (size_t)n);
   double* Y = bp + seg(8);
-  const int npan = (n - 1 + ZWB - 1) / ZWB;
-  double* tws = Y + seg((size_t)n * n) + seg(2 * (size_t)std::max(npan, 1) * ZWB * ZWB);
+  double* tws = Y + seg((size_t)n * n) + zback_extra_doubles(n, 1);
   zprep_tri_kernel<<<1, 1024, 0, st>>>(reinterpret_cast<const zc*>(evd), dvim, n, dg, off, ph, bp);
   cudaError_t e = launch_zbisect(dg, off, n, 1, bp, mu, vals_im, st);
   if (e != cudaSuccess || !Vd) return e;

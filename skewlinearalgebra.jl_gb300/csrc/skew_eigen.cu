@@ -36,6 +36,7 @@
 #include "skew_common.cuh"
 #include "skew_internal.h"
 #include "skew_twisted.cuh"
+#include "skew_back.cuh"
 #include "skew_funcs.cuh"
 #include "skew_oz.cuh"
 
@@ -539,8 +540,9 @@ __global__ void __launch_bounds__(ENT) eigen_back_kernel(EigenBatch E) {
   __shared__ int s_next;
   __shared__ double T[EB * EB], P[32], scratch[ENW * 32];
   extern __shared__ __align__(16) double esm[];  // Vs (nmax x EB, row-major) | Zs (EB x 2 nmax)
+  const int nmax = min(E.nmax, kBackOzMin);
   double* Vs = esm;
-  double* Zs = esm + (size_t)E.nmax * EB;
+  double* Zs = esm + (size_t)nmax * EB;
   __shared__ int s_chunk;
   for (;;) {
     // work item: (matrix in the processing order, chunk of kBackCols columns), the
@@ -957,9 +959,42 @@ cudaError_t launch_copy_ev(const double* const* ev_in, const int32_t* n, const i
   return cudaGetLastError();
 }
 
-size_t eigen_work_doubles(int n) {
+// Back-transformation of the batch on the tensor cores from n = kBackOzMin: its workspace
+// lies in work blocks 1 and 2 (block 0 holds Q, block 3 its metadata) where it fits, else
+// behind the four blocks.
+static size_t base_work_doubles(int n) {
   return (size_t)std::max<int64_t>(4 * (int64_t)n * n, fallback_ws_doubles(n));
 }
+__host__ __device__ inline size_t batch_back_doubles(int n) { return back_ws_doubles<false>(n, n - 2, 2 * n, 1); }
+size_t eigen_work_doubles(int n) {
+  const size_t base = base_work_doubles(n);
+  if (n < kBackOzMin || batch_back_doubles(n) <= 2 * (size_t)n * n) return base;
+  return base + batch_back_doubles(n);
+}
+
+struct BatchBack {
+  EigenBatch E;
+  __device__ bool get(int b, BackTask<false>& T) const {
+    const int n = E.n[b];
+    if (n < kBackOzMin || E.status[b] == SKEW_NO_CONVERGENCE) return false;
+    const bool qonly = E.back_q && E.fsel && E.fsel[b] == 1;
+    T.A = E.refl[b];
+    T.lda = n;
+    T.tau = E.tau + E.off_n[b];
+    T.n = n;
+    T.nref = n - 2;
+    T.X[0] = qonly ? E.pwork[b] : E.Vr[b];
+    T.X[1] = E.Vi[b];
+    T.nc[0] = n;
+    T.nc[1] = qonly ? 0 : n;
+    T.ldx = n;
+    T.status = E.status + b;
+    const size_t nn = (size_t)n * n;
+    back_ws_set(T, E.pwork[b] + (batch_back_doubles(n) <= 2 * nn ? nn : (size_t)max((int64_t)(4 * nn), fallback_ws_doubles(n))), 2 * n, 1);
+    return true;
+  }
+};
+
 
 __global__ void gather_ev_kernel(const double* __restrict__ ev, const int64_t* __restrict__ off_n,
                                  const int32_t* __restrict__ idx, int n, double* __restrict__ e_g) {
@@ -989,15 +1024,20 @@ cudaError_t launch_eigen_vectors(const EigenBatch& E, int grid, cudaStream_t st)
   return cudaGetLastError();
 }
 
+// Matrices below kBackOzMin: reflector blocks of 8 on the FP64 pipe, items of column
+// chunks; from it on, panels on the tensor cores (skew_back.cuh), all matrices at a time.
 cudaError_t launch_eigen_back(const EigenBatch& E, int grid, int nmax, cudaStream_t st) {
-  cudaError_t e = cudaMemsetAsync(E.counter, 0, sizeof(unsigned), st);
-  if (e != cudaSuccess) return e;
-  const size_t smem = sizeof(double) * (size_t)EB * 3 * (size_t)nmax;
-  static std::atomic<uint64_t> raised{0};
-  e = raise_smem_limit_once((const void*)eigen_back_kernel, raised);
-  if (e != cudaSuccess) return e;
-  eigen_back_kernel<<<grid, ENT, smem, st>>>(E);
-  return cudaGetLastError();
+  cudaError_t e;
+  if (E.back_items > 0) {
+    e = cudaMemsetAsync(E.counter, 0, sizeof(unsigned), st);
+    if (e != cudaSuccess) return e;
+    const size_t smem = sizeof(double) * (size_t)EB * 3 * (size_t)std::min(nmax, kBackOzMin);
+    eigen_back_kernel<<<grid, ENT, smem, st>>>(E);
+    if ((e = cudaGetLastError())) return e;
+  }
+  if (nmax < kBackOzMin) return cudaSuccess;
+  BatchBack S{E};
+  return back_transform_oz<false>(S, E.count, nmax, nmax - 2, 2 * nmax, 1, st);
 }
 
 // ---------------------------------------------------------------------------

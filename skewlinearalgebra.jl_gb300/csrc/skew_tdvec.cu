@@ -23,8 +23,7 @@
 //      pattern (real on odd 1-based rows, imaginary on even rows, sign flipped
 //      every pair); the vector of -sigma_k is the conjugate of that of sigma_k;
 //   5. back-transformation X <- Q X with the stored reflectors, panel by panel in
-//      compact WY form (Q_b = I - V T V^T, dlarft-style T), each CTA owning a
-//      strip of 32 columns (no inter-CTA dependence);
+//      compact WY form on the tensor cores (skew_back.cuh);
 //   6. the +sigma columns are mirrored from the -sigma columns (Vr equal, Vi
 //      negated).
 #include <cuda_runtime.h>
@@ -33,21 +32,19 @@
 
 #include <algorithm>
 
-#include "skew_common.cuh"
 #include "skew_internal.h"
+#include "skew_back.cuh"
+#include "skew_common.cuh"
 #include "skew_twisted.cuh"
 
 namespace skew {
 
 constexpr int TW_NT = 64;  // threads per CTA of the twisted kernel (one vector each)
 constexpr int LW = 16;     // half-width of the Lowdin band
-constexpr int WB = 64;     // reflectors per compact-WY panel
-constexpr int SW = 32;     // columns per back-transformation strip
 constexpr int RC = 32;     // rows per staged chunk
 
 struct TdvecLayout {
   int n, h, K, KP;  // n, positive eigenvalues, vectors (h + n odd), padded to 32
-  int npan;         // WY panels
   int full;         // 1: general symmetric tridiagonal (diagonal dg), one vector per eigenvalue (K = n)
   const double* dg; // diagonal (full mode) or null (zero diagonal)
   // batches of equal-size problems (full mode): problem mb = blockIdx.z uses the
@@ -59,7 +56,6 @@ struct TdvecLayout {
   double* nrm2;     // KP
   double* bandU;    // KP x (LW + 1) raw dots over even rows
   double* bandV;    // KP x (LW + 1) raw dots over odd rows
-  double* T;        // npan x WB x WB
   // gate != null: every kernel of the pipeline returns at once unless *gate ==
   // gate_on (two pipelines are queued and the device picks one, no host sync)
   const int* gate;
@@ -82,7 +78,6 @@ static TdvecLayout layout(int n, double* ws, bool full = false, const double* dg
   L.dg = dg;
   L.mstride = large_eigen_ws_doubles(n);
   L.KP = (L.K + 31) / 32 * 32;
-  L.npan = (n - 2 + WB - 1) / WB;
   const size_t big = (size_t)n * L.KP;
   L.dp = ws;
   L.dm = L.dp + big;
@@ -90,7 +85,6 @@ static TdvecLayout layout(int n, double* ws, bool full = false, const double* dg
   L.nrm2 = L.z + big;
   L.bandU = L.nrm2 + L.KP;
   L.bandV = L.bandU + (size_t)L.KP * (LW + 1);
-  L.T = L.bandV + (size_t)L.KP * (LW + 1);
   L.gate = nullptr;
   L.gate_on = 0;
   return L;
@@ -98,8 +92,7 @@ static TdvecLayout layout(int n, double* ws, bool full = false, const double* dg
 
 size_t large_eigen_ws_doubles(int n) {
   const int KP = (n + 31) / 32 * 32;  // covers both modes (K <= n)
-  const int npan = (n - 2 + WB - 1) / WB;
-  return 3 * (size_t)n * KP + KP + 2 * (size_t)KP * (LW + 1) + (size_t)std::max(npan, 1) * WB * WB + 64;
+  return 3 * (size_t)n * KP + KP + 2 * (size_t)KP * (LW + 1) + 64;
 }
 
 // the layout of problem mb of a batch (mb = 0: unchanged)
@@ -112,7 +105,6 @@ __device__ __forceinline__ TdvecLayout at_problem(TdvecLayout L, int mb) {
   L.nrm2 += o;
   L.bandU += o;
   L.bandV += o;
-  L.T += o;
   if (L.dg) L.dg += (size_t)mb * L.n;
   return L;
 }
@@ -381,221 +373,18 @@ cudaError_t symtri_vectors(const double* dg, const double* e, int n, const doubl
 }
 
 // ---------------------------------------------------------------------------
-// 5. compact WY factors T_b (dlarft, forward, columnwise) of each panel
+// 5. X <- Q X (skew_back.cuh): one matrix, its columns in two groups
 // ---------------------------------------------------------------------------
-// Reflector c (0 <= c <= n-3) lives in column c of A below the diagonal: v_c = 0
-// above row c+1, v_c[c+1] = 1, v_c[c+2:] = A[c+2:, c]; tau_c = 0 means H_c = I.
-__device__ __forceinline__ double refl_at(const double* A, int64_t lda, const double* tau, int row, int c) {
-  if (row < c + 1 || tau[c] == 0.0) return 0.0;
-  return (row == c + 1) ? 1.0 : A[row + (int64_t)c * lda];
-}
-
-constexpr int WT_NT = 256;
-constexpr int WT_RC = 16;  // rows per staged chunk of the factor kernel
-
-// One array holds both: the lower triangle of M is the Gram matrix G = V^T V
-// (symmetric, so G(l, i) is read as M(i, l)), the upper triangle and diagonal
-// receive T as the recurrence produces it (a diagonal G entry is never needed).
-__global__ void __launch_bounds__(WT_NT) wy_factor_kernel(const double* __restrict__ A, int64_t lda,
-                                                          const double* __restrict__ tau, TdvecLayout L) {
-  if (gated_off(L)) return;
-  __shared__ double Vs[WT_RC][WB + 1];
-  __shared__ double M[WB][WB + 1];
-  const int b = blockIdx.x;
-  const int n = L.n;
-  const int c0 = b * WB, c1 = min(c0 + WB, n - 2), nb = c1 - c0;
-  const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
-  double acc[4][4];
-#pragma unroll
-  for (int a = 0; a < 4; a++)
-#pragma unroll
-    for (int q = 0; q < 4; q++) acc[a][q] = 0.0;
-  for (int r0 = c0 + 1; r0 < n; r0 += WT_RC) {
-    __syncthreads();
-    for (int idx = threadIdx.x; idx < WT_RC * WB; idx += WT_NT) {
-      const int cc = idx / WT_RC, rr = idx - cc * WT_RC;
-      const int row = r0 + rr, c = c0 + cc;
-      Vs[rr][cc] = (row < n && cc < nb) ? refl_at(A, lda, tau, row, c) : 0.0;
-    }
-    __syncthreads();
-#pragma unroll 4
-    for (int rr = 0; rr < WT_RC; rr++) {
-      double va[4], vb[4];
-#pragma unroll
-      for (int a = 0; a < 4; a++) {
-        va[a] = Vs[rr][ty + 16 * a];
-        vb[a] = Vs[rr][tx + 16 * a];
-      }
-#pragma unroll
-      for (int a = 0; a < 4; a++)
-#pragma unroll
-        for (int q = 0; q < 4; q++) acc[a][q] = fma(va[a], vb[q], acc[a][q]);
-    }
+struct LargeBack {
+  BackTask<false> B;
+  const int* gate;
+  int gate_on;
+  __device__ bool get(int, BackTask<false>& T) const {
+    if (gate && *gate != gate_on) return false;
+    T = B;
+    return true;
   }
-  __syncthreads();
-#pragma unroll
-  for (int a = 0; a < 4; a++)
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-      const int i = ty + 16 * a, j = tx + 16 * q;
-      M[i][j] = (i > j) ? acc[a][q] : 0.0;  // G below the diagonal, T (zero so far) on and above
-    }
-  __syncthreads();
-  // T(i,i) = tau_i; T(0:i, i) = -tau_i T(0:i, 0:i) G(0:i, i)
-  for (int i = 0; i < nb; i++) {
-    const double ti = tau[c0 + i];
-    if (threadIdx.x < i) {
-      const int j = threadIdx.x;
-      double s = 0.0;
-      for (int l = j; l < i; l++) s = fma(M[j][l], M[i][l], s);
-      M[j][i] = neg(ti) * s;
-    }
-    if (threadIdx.x == 0) M[i][i] = ti;
-    __syncthreads();
-  }
-  double* Tg = L.T + (size_t)b * WB * WB;
-  for (int idx = threadIdx.x; idx < WB * WB; idx += WT_NT) {
-    const int i = idx / WB, j = idx % WB;
-    Tg[idx] = (j >= i) ? M[i][j] : 0.0;
-  }
-}
-
-// ---------------------------------------------------------------------------
-// 5. X <- Q X, one CTA per strip of SW columns, panels last to first:
-//    W = V^T X, W <- T W, X <- X - V W
-// ---------------------------------------------------------------------------
-constexpr int BT_NT = 256;
-
-struct StripParams {
-  const double* A;
-  int64_t lda;
-  const double* tau;
-  TdvecLayout L;
-  double* Xr;  // columns [cr0, n) of Vr
-  double* Xi;  // columns [ci0, n) of Vi
-  int64_t ldv;
-  int cr0, ci0, nstr_r;  // strips over Vr first
 };
-
-__global__ void __launch_bounds__(BT_NT) back_strip_kernel(StripParams P) {
-  if (gated_off(P.L)) return;
-  extern __shared__ __align__(16) double bsm[];
-  double(*Ts)[WB + 1] = reinterpret_cast<double(*)[WB + 1]>(bsm);                   // WB x (WB+1)
-  double(*Ws)[SW + 1] = reinterpret_cast<double(*)[SW + 1]>(bsm + WB * (WB + 1));  // WB x (SW+1)
-  double(*Vs)[WB + 1] = reinterpret_cast<double(*)[WB + 1]>(bsm + WB * (WB + 1) + WB * (SW + 1));  // RC x (WB+1)
-  double(*Xs)[SW + 1] =
-      reinterpret_cast<double(*)[SW + 1]>(bsm + WB * (WB + 1) + WB * (SW + 1) + RC * (WB + 1));  // RC x (SW+1)
-  const int n = P.L.n;
-  const int s = blockIdx.x;
-  double* X;
-  int col0, ncol;
-  if (s < P.nstr_r) {
-    X = P.Xr;
-    col0 = P.cr0 + s * SW;
-  } else {
-    X = P.Xi;
-    col0 = P.ci0 + (s - P.nstr_r) * SW;
-  }
-  ncol = min(SW, n - col0);
-  X += (int64_t)col0 * P.ldv;
-  const int64_t ldx = P.ldv;
-  // thread tiles: W (WB x SW = 64 x 32): 4 x 2 per thread; X chunk (RC x SW = 32 x 32): 2 x 2 per thread
-  const int wr = (threadIdx.x >> 4) * 4, wc = (threadIdx.x & 15) * 2;
-  const int xr = (threadIdx.x >> 4) * 2, xc = (threadIdx.x & 15) * 2;
-  for (int b = P.L.npan - 1; b >= 0; b--) {
-    const int c0 = b * WB, c1 = min(c0 + WB, n - 2), nb = c1 - c0;
-    __syncthreads();
-    for (int idx = threadIdx.x; idx < WB * WB; idx += BT_NT)
-      Ts[idx / WB][idx % WB] = P.L.T[(size_t)b * WB * WB + idx];
-    // W = V^T X over rows c0+1 .. n-1
-    double w[4][2];
-#pragma unroll
-    for (int a = 0; a < 4; a++) w[a][0] = w[a][1] = 0.0;
-    for (int r0 = c0 + 1; r0 < n; r0 += RC) {
-      __syncthreads();
-      for (int idx = threadIdx.x; idx < RC * WB; idx += BT_NT) {
-        const int cc = idx / RC, rr = idx - cc * RC;
-        const int row = r0 + rr;
-        Vs[rr][cc] = (row < n && cc < nb) ? refl_at(P.A, P.lda, P.tau, row, c0 + cc) : 0.0;
-      }
-      for (int idx = threadIdx.x; idx < RC * SW; idx += BT_NT) {
-        const int cc = idx / RC, rr = idx - cc * RC;
-        const int row = r0 + rr;
-        Xs[rr][cc] = (row < n && cc < ncol) ? X[row + (int64_t)cc * ldx] : 0.0;
-      }
-      __syncthreads();
-#pragma unroll 8
-      for (int rr = 0; rr < RC; rr++) {
-        const double x0 = Xs[rr][wc], x1 = Xs[rr][wc + 1];
-#pragma unroll
-        for (int a = 0; a < 4; a++) {
-          const double v = Vs[rr][wr + a];
-          w[a][0] = fma(v, x0, w[a][0]);
-          w[a][1] = fma(v, x1, w[a][1]);
-        }
-      }
-    }
-#pragma unroll
-    for (int a = 0; a < 4; a++) {
-      Ws[wr + a][wc] = w[a][0];
-      Ws[wr + a][wc + 1] = w[a][1];
-    }
-    __syncthreads();
-    // W <- T W (T upper triangular)
-    double tw[4][2];
-#pragma unroll
-    for (int a = 0; a < 4; a++) {
-      tw[a][0] = tw[a][1] = 0.0;
-      const int i = wr + a;
-      for (int l = i; l < WB; l++) {
-        const double t = Ts[i][l];
-        tw[a][0] = fma(t, Ws[l][wc], tw[a][0]);
-        tw[a][1] = fma(t, Ws[l][wc + 1], tw[a][1]);
-      }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int a = 0; a < 4; a++) {
-      Ws[wr + a][wc] = tw[a][0];
-      Ws[wr + a][wc + 1] = tw[a][1];
-    }
-    // X <- X - V W over rows c0+1 .. n-1 (X chunk staged: coalesced column reads and writes)
-    for (int r0 = c0 + 1; r0 < n; r0 += RC) {
-      __syncthreads();
-      for (int idx = threadIdx.x; idx < RC * WB; idx += BT_NT) {
-        const int cc = idx / RC, rr = idx - cc * RC;
-        const int row = r0 + rr;
-        Vs[rr][cc] = (row < n && cc < nb) ? refl_at(P.A, P.lda, P.tau, row, c0 + cc) : 0.0;
-      }
-      for (int idx = threadIdx.x; idx < RC * SW; idx += BT_NT) {
-        const int cc = idx / RC, rr = idx - cc * RC;
-        const int row = r0 + rr;
-        Xs[rr][cc] = (row < n && cc < ncol) ? X[row + (int64_t)cc * ldx] : 0.0;
-      }
-      __syncthreads();
-      double acc[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
-#pragma unroll 8
-      for (int l = 0; l < WB; l++) {
-        const double w0 = Ws[l][xc], w1 = Ws[l][xc + 1];
-        const double v0 = Vs[xr][l], v1 = Vs[xr + 1][l];
-        acc[0][0] = fma(v0, w0, acc[0][0]);
-        acc[0][1] = fma(v0, w1, acc[0][1]);
-        acc[1][0] = fma(v1, w0, acc[1][0]);
-        acc[1][1] = fma(v1, w1, acc[1][1]);
-      }
-#pragma unroll
-      for (int a = 0; a < 2; a++)
-#pragma unroll
-        for (int q = 0; q < 2; q++) Xs[xr + a][xc + q] -= acc[a][q];
-      __syncthreads();
-      for (int idx = threadIdx.x; idx < RC * SW; idx += BT_NT) {
-        const int cc = idx / RC, rr = idx - cc * RC;
-        const int row = r0 + rr;
-        if (row < n && cc < ncol) X[row + (int64_t)cc * ldx] = Xs[rr][cc];
-      }
-    }
-  }
-}
 
 // 6. +sigma columns: Vr[:, k] = Vr[:, n-1-k], Vi[:, k] = -Vi[:, n-1-k]; odd n: Vi[:, h] = 0
 __global__ void mirror_kernel(double* __restrict__ Vr, double* __restrict__ Vi, int64_t ldv, int n,
@@ -612,10 +401,6 @@ __global__ void mirror_kernel(double* __restrict__ Vr, double* __restrict__ Vi, 
       Vi[i + (int64_t)h * ldv] = 0.0;  // k == h only launched for odd n
     }
   }
-}
-
-static size_t strip_smem_bytes() {
-  return sizeof(double) * ((size_t)WB * (WB + 1) + (size_t)WB * (SW + 1) + (size_t)RC * (WB + 1) + (size_t)RC * (SW + 1));
 }
 
 // Batched skew-mode write and mirror for G problems of one size (per-problem output
@@ -810,29 +595,34 @@ __global__ void __launch_bounds__(LA_NT) tdvec_write_fallback_batch_kernel(Tdvec
   }
 }
 
+// Strips of 32 columns per CTA walking all panels on the FP64 pipe took 43.5 ms at
+// n = 2048; panel by panel on the tensor cores 2.8 ms.  The vectors are in Vr and Vi, so
+// the workspace of the twisted kernels (3 n KP doubles of the full mode) is free.
 static cudaError_t back_transform(const double* A, int64_t lda, const double* tau, const TdvecLayout& L, double* Vr,
-                                  double* Vi, int64_t ldv, int cr0, int ci0, cudaStream_t st) {
+                                  double* Vi, int64_t ldv, int cr0, int ci0, double* ws, cudaStream_t st) {
   const int n = L.n;
-  wy_factor_kernel<<<L.npan, WT_NT, 0, st>>>(A, lda, tau, L);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  StripParams P;
-  P.A = A;
-  P.lda = lda;
-  P.tau = tau;
-  P.L = L;
-  P.Xr = Vr;
-  P.Xi = Vi;
-  P.ldv = ldv;
-  P.cr0 = cr0;
-  P.ci0 = ci0;
-  P.nstr_r = (n - cr0 + SW - 1) / SW;
-  const int nstr_i = (n - ci0 + SW - 1) / SW;
-  static std::atomic<uint64_t> raised{0};
-  e = raise_smem_limit_once((const void*)back_strip_kernel, raised);
-  if (e != cudaSuccess) return e;
-  back_strip_kernel<<<P.nstr_r + nstr_i, BT_NT, strip_smem_bytes(), st>>>(P);
-  return cudaGetLastError();
+  int dev = 0, sms = 148;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  LargeBack S;
+  S.B.A = A;
+  S.B.lda = lda;
+  S.B.tau = tau;
+  S.B.n = n;
+  S.B.nref = n - 2;
+  S.B.X[0] = Vr + (int64_t)cr0 * ldv;
+  S.B.X[1] = Vi + (int64_t)ci0 * ldv;
+  S.B.ldx = ldv;
+  S.B.nc[0] = n - cr0;
+  S.B.nc[1] = n - ci0;
+  S.B.status = nullptr;
+  S.gate = L.gate;
+  S.gate_on = L.gate_on;
+  const int cols = S.B.nc[0] + S.B.nc[1];
+  const size_t room = 3 * (size_t)n * ((n + 31) / 32 * 32);
+  int splits = back_splits(cols, 1, sms);
+  while (splits > 1 && back_ws_doubles<false>(n, n - 2, cols, splits) > room) splits /= 2;
+  back_ws_set(S.B, ws, cols, splits);
+  return back_transform_oz<false>(S, 1, n, n - 2, cols, splits, st);
 }
 
 size_t large_eigen_aux_doubles(int n) { return (size_t)n + 8; }
@@ -860,7 +650,7 @@ cudaError_t large_eigen_vectors(const double* A, int64_t lda, int n, const doubl
   if (e != cudaSuccess) return e;
   if (A) {  // A == null: a tridiagonal input, Q = I
     // -sigma columns and the zero vector of Vr, -sigma columns of Vi
-    e = back_transform(A, lda, tau, L, Vr, Vi, ldv, L.h, L.h + (n & 1), st);
+    e = back_transform(A, lda, tau, L, Vr, Vi, ldv, L.h, L.h + (n & 1), ws, st);
     if (e != cudaSuccess) return e;
   }
   mirror_kernel<<<dim3((n + 255) / 256, L.h + (n & 1)), 256, 0, st>>>(Vr, Vi, ldv, n, gate);
@@ -877,7 +667,7 @@ cudaError_t large_eigen_vectors(const double* A, int64_t lda, int n, const doubl
   tdvec_write_fallback_kernel<<<dim3(F.KP / 32, (n + RC - 1) / RC), LA_NT, 0, st>>>(F, X, Vr, Vi, ldv);
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  if (A) return back_transform(A, lda, tau, F, Vr, Vi, ldv, 0, 0, st);
+  if (A) return back_transform(A, lda, tau, F, Vr, Vi, ldv, 0, 0, ws, st);
   return cudaSuccess;
 }
 
