@@ -311,11 +311,15 @@ static int single(skew_handle_t h, double* A, int64_t n, int64_t lda, double* G,
   return SKEW_OK;
 }
 
+static size_t reduce_ws_doubles(int64_t n) {
+  return std::max(blocked_ws_doubles((int)n) + persist_ws_extra_doubles(), wide_ws_doubles((int)n));
+}
+
 // Blocked reduction of a large matrix into tau/ev (device); A in place.
 static int blocked(skew_handle_t h, double* A, int64_t n, int64_t lda, double* tau, double* ev, int* info,
                    size_t extra_doubles, double** extra) {
   if (!h || !A || lda < n || n > (1LL << 15)) return n > (1LL << 15) ? SKEW_UNSUPPORTED : SKEW_BAD_ARG;
-  const size_t wsd = blocked_ws_doubles((int)n) + persist_ws_extra_doubles();
+  const size_t wsd = reduce_ws_doubles(n);
   int st = ensure_ws(h, sizeof(double) * (wsd + extra_doubles));
   if (st) return st;
   double* ws = (double*)h->ws;
@@ -332,6 +336,14 @@ static int blocked(skew_handle_t h, double* A, int64_t n, int64_t lda, double* t
     cudaError_t e = cluster_hessenberg(A, lda, (int)n, tau, ev, info, h->stream);
     if (e == cudaSuccess) return SKEW_OK;
     if (e != cudaErrorNotSupported) return SKEW_CUDA_ERROR;
+    cudaGetLastError();
+  }
+  // above kWideMin: the panel's product in fixed point, the trailing update on the
+  // tensor cores
+  if (n > kWideMin && h->tune.blocked_persistent != 0) {
+    cudaError_t e = wide_hessenberg(A, lda, (int)n, tau, ev, info, ws, h->sms, h->tune, h->stream);
+    if (e == cudaSuccess) return SKEW_OK;
+    if (e != cudaErrorNotSupported && e != cudaErrorCooperativeLaunchTooLarge) return SKEW_CUDA_ERROR;
     cudaGetLastError();
   }
   // one cooperative launch for all panels when v fits in shared memory; the
@@ -361,7 +373,7 @@ int skew_logabspf_d(skew_handle_t h, double* A, int64_t n, int64_t lda, double* 
   if (n >= blocked_min_n(h) && (n % 2) == 0) {
     double* extra = nullptr;
     // workspace layout: [blocked ws][ev (n)][tau (n)][not-skew flag]; size it before the check
-    const size_t wsd = blocked_ws_doubles((int)n) + persist_ws_extra_doubles();
+    const size_t wsd = reduce_ws_doubles(n);
     int st = ensure_ws(h, sizeof(double) * (wsd + 2 * (size_t)n + 1));
     if (st) return st;
     double* flag = (double*)h->ws + wsd + 2 * (size_t)n;  // after blocked()'s ev/tau extra area
@@ -1263,7 +1275,7 @@ static int single_func(skew_handle_t h, double* A, int64_t n, int64_t lda, doubl
 static int eigen_large(skew_handle_t h, double* A, int64_t n, int64_t lda, double* vals_im, double* Vr, double* Vi,
                        int64_t ldv, int* info) {
   if (lda < n || ldv < n || n > (1LL << 15)) return n > (1LL << 15) ? SKEW_UNSUPPORTED : SKEW_BAD_ARG;
-  const size_t wsd = blocked_ws_doubles((int)n) + persist_ws_extra_doubles();
+  const size_t wsd = reduce_ws_doubles(n);
   const size_t lwsd = large_eigen_ws_doubles((int)n), auxd = large_eigen_aux_doubles((int)n);
   const size_t extra = 2 * (size_t)n + 8 + lwsd + auxd + 1;
   int st = ensure_ws(h, sizeof(double) * (wsd + extra));

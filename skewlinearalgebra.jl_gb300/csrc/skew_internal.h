@@ -300,6 +300,14 @@ cudaError_t launch_eigen_func(const EigenBatch& E, int mode, cudaStream_t st);
 // exp adjoint: the real Schur basis Q (and fsel) from vals, Vr, Vi into pwork
 cudaError_t launch_schur_basis(const EigenBatch& E, cudaStream_t st);
 
+// One real matrix with n > kWideMin (skew_wide.cu): the product of the panel in fixed point,
+// the trailing update on the tensor cores.  cudaErrorNotSupported (nothing done) where it
+// cannot run; the caller then takes the kernels below.
+constexpr int kWideMin = 1024;
+size_t wide_ws_doubles(int n);
+cudaError_t wide_hessenberg(double* A, int64_t lda, int n, double* tau, double* ev, int* info, double* ws, int sms,
+                            const Tuning& T, cudaStream_t st);
+
 // Multi-CTA blocked reduction of one large matrix (skew_blocked.cu).
 size_t blocked_ws_doubles(int n);
 cudaError_t blocked_hessenberg(double* A, int64_t lda, int n, double* tau, double* ev, int* info, double* ws, int sms,
