@@ -794,6 +794,7 @@ int skew_batch_eigvals_d(skew_batch_plan_t P, const double* const* A, double* co
     tp.fallback = P->d_fallback;
     tp.grid = (int)std::min<int64_t>(2 * (int64_t)P->h->sms, P->count);
     tp.max_iter = P->h->tune.qr_max_iter;
+    tp.nmax = *std::max_element(P->n_host.begin(), P->n_host.end());
     CK(launch_batch_trieig(tp, P->h->stream));
     return SKEW_OK;
   });
@@ -1854,6 +1855,7 @@ static int tridiag_qr_vals(skew_handle_t h, const double* ev, int64_t n, double*
   tp.fallback = P->d_fallback;
   tp.grid = 1;
   tp.max_iter = h->tune.qr_max_iter;
+  tp.nmax = (int)n;
   CK(launch_batch_trieig(tp, h->stream));
   return SKEW_OK;
 }

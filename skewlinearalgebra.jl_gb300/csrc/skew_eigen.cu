@@ -37,6 +37,7 @@
 #include "skew_internal.h"
 #include "skew_twisted.cuh"
 #include "skew_back.cuh"
+#include "skew_chain.cuh"
 #include "skew_funcs.cuh"
 #include "skew_oz.cuh"
 
@@ -96,135 +97,42 @@ __device__ void reducetozero_g(double* ev, double* G, int n) {
   if (n == 2) ev[1] = __dadd_rn(__dmul_rn(s, a), __dmul_rn(b, c));
 }
 
-// implicitstep_vec! (skeweigen.jl:158-193) without the vector update: the
-// rotations (c, s) of steps i = start..n-1 are appended to log after a header
-// (start, n).  Returns the new start, or -1 if the log is full.  As in the
-// reference, a split found mid-sweep moves `start` at once, so the next step
-// restarts the shifted rotation from there (the replay needs only i, not start).
-__device__ int implicitstep_log(double* ev, int n, int start, double* log, int64_t& len, int64_t cap) {
-  if (len + 2 + 2 * (int64_t)(n - start) > cap) return -1;
-  log[len++] = (double)start;
-  log[len++] = (double)n;
-  double bulge = 0.0;
-  const double shift = __dmul_rn(ev[n - 1], ev[n - 1]);
-  const double tol = 10.0 * 2.220446049250313e-16;
-  const int first = start;
-  // ev[i-2], ev[i-1], ev[i] of step i are what step i-1 wrote: carried in
-  // registers; ev[i+1] (untouched this sweep) is loaded one step ahead.  Every
-  // store of the reference's step is still made.
-  double pa = 0.0;            // ev[i-2] as left by the previous step
-  double b = ev[first - 1];   // ev[i-1]
-  double g = ev[first];       // ev[i]
-  double z = (first < n - 1) ? ev[first + 1] : 0.0;
-  for (int i = first; i <= n - 1; i++) {
-    const double zn = (i + 2 <= n - 1) ? ev[i + 2] : 0.0;
-    const double a = (i > start ? pa : 0.0);
-    double c, s;
-    if (i > start) {
-      givens_e(a, bulge, c, s);
-    } else {
-      const double x1 = __dadd_rn(__dsub_rn(neg(__dmul_rn(a, a)), __dmul_rn(b, b)), shift);
-      const double x2 = __dadd_rn(neg(__dmul_rn(a, bulge)), __dmul_rn(b, g));
-      givens_e(x1, x2, c, s);
+// The iteration of skewtrieigen_divided! (skewtrieigen_merged! without the mem deflation),
+// four lanes per matrix (skew_chain.cuh); the replay needs only each sweep's header and
+// rotations.
+__global__ void __launch_bounds__(32) eigen_chain_kernel(EigenBatch E) {
+  extern __shared__ double chain_ev[];
+  const int t = blockIdx.x * CH_M + threadIdx.x / CH_G, g = threadIdx.x & (CH_G - 1);
+  const int stride = min(E.nmax, E.chain_nmax) | 1;
+  double* ev = chain_ev + (threadIdx.x / CH_G) * stride;
+  Chain<true> S;
+  S.run = false;
+  S.status = SKEW_OK;
+  S.len = 0;
+  int b = 0, N = 0;
+  if (t < E.count) {
+    b = E.order[t];
+    N = E.n[b];
+    if (N > E.chain_nmax) {  // eigenpairs from bisection and twisted vectors instead
+      if (g == 0) E.status[b] = SKEW_OK;
+      N = -1;
     }
-    if (i > 1) ev[i - 2] = __dadd_rn(__dmul_rn(c, a), __dmul_rn(s, bulge));
-    const double nb = __dsub_rn(__dmul_rn(c, b), __dmul_rn(s, g));
-    const double ng = __dadd_rn(__dmul_rn(s, b), __dmul_rn(c, g));
-    ev[i - 1] = nb;
-    ev[i] = ng;
-    if (i < n - 1) {
-      const double nz = __dmul_rn(z, c);
-      ev[i + 1] = nz;
-      bulge = __dmul_rn(s, z);
-      if (fabs(bulge) < tol && fabs(nb) < tol) start = i + 1;
-      pa = nb;
-      b = ng;
-      g = nz;
-      z = zn;
-    }
-    log[len++] = c;
-    log[len++] = s;
+    const double* src = E.ev + E.off_n[b];
+    double* keep = E.evb + E.off_n[b];
+    for (int i = g; i + 1 < N; i += CH_G) ev[i] = keep[i] = src[i];
+    for (int i = g; i < N; i += CH_G) E.vals[b][i] = 0.0;
   }
-  return start;
-}
-
-__global__ void eigen_chain_kernel(EigenBatch E) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= E.count) return;
-  const int b = E.order[t];
-  const int N = E.n[b];
-  if (N > E.chain_nmax) {  // eigenpairs from bisection and twisted vectors instead
-    E.status[b] = SKEW_OK;
-    return;
+  __syncwarp();
+  if (N >= 2 && (N & 1) && g == 0) reducetozero_g(ev, E.G + E.off_n[b], N - 1);
+  __syncwarp();
+  S.nb = S.bulge = S.q1 = S.q2 = S.shift = 0.0;
+  S.i = S.m = S.start = 0;
+  if (N >= 2) S.begin(ev, N & ~1, E.vals[b], E.max_iter, E.merged, E.log + E.off_log[b], E.cap_log[b]);
+  while (__any_sync(0xffffffffu, S.run)) S.step();
+  if (N >= 0 && t < E.count && g == 0) {
+    E.log_len[b] = S.len;
+    E.status[b] = S.status;
   }
-  double* ev = E.ev + E.off_n[b];
-  double* evb = E.evb + E.off_n[b];
-  double* G = E.G + E.off_n[b];
-  double* vals = E.vals[b];
-  double* log = E.log + E.off_log[b];
-  const int64_t cap = E.cap_log[b];
-  int64_t len = 0;
-  for (int i = 0; i + 1 < N; i++) evb[i] = ev[i];
-  for (int i = 0; i < N; i++) vals[i] = 0.0;
-  int status = SKEW_OK;
-  int n = N;
-  if (N >= 2) {
-    if (n & 1) {
-      n -= 1;
-      reducetozero_g(ev, G, n);
-    }
-    const double tol = 10.0 * 2.220446049250313e-16;
-    const int max_iter = E.max_iter > 0 ? E.max_iter : 30 * n;
-    int iter = 0, count_static = 0, start = 1;
-    double mem = 1.0;
-    while (n > 2 && iter < max_iter) {
-      start = implicitstep_log(ev, n - 1, start, log, len, cap);
-      if (start < 0) {
-        status = SKEW_NO_CONVERGENCE;
-        break;
-      }
-      while (n > 2 && fabs(ev[n - 2]) <= tol) {
-        vals[n - 1] = 0.0;
-        n -= 1;
-      }
-      while (n > 2 && fabs(ev[n - 3]) <= tol * fabs(ev[n - 2])) {
-        vals[n - 2] = ev[n - 2];
-        vals[n - 1] = neg(ev[n - 2]);
-        n -= 2;
-      }
-      if (!E.merged && n > 2 && fabs(ev[n - 2] - mem) < tol) {  // skeweigen.jl:355-358 (divided only)
-        vals[n - 2] = ev[n - 2];
-        vals[n - 1] = neg(ev[n - 2]);
-        n -= 2;
-      }
-      if (start > n - 2) start = 1;
-      if (n > 1 && fabs(mem - ev[n - 2]) < 0.0001 * fabs(ev[n - 2])) {
-        count_static += 1;
-        if (count_static > 4) {
-          status = SKEW_FALLBACK_USED;
-          break;
-        }
-      } else {
-        count_static = 0;
-      }
-      mem = (n > 1 ? ev[n - 2] : 0.0);
-      iter += 1;
-    }
-    if (status == SKEW_OK) {
-      if (n > 2) {
-        status = SKEW_NO_CONVERGENCE;
-      } else if (n == 2) {
-        vals[0] = ev[0];
-        vals[1] = neg(ev[0]);
-      } else if (n == 1) {
-        vals[0] = 0.0;
-      }
-    }
-  } else if (N == 1) {
-    vals[0] = 0.0;
-  }
-  E.log_len[b] = len;
-  E.status[b] = status;
 }
 
 // ---------------------------------------------------------------------------
@@ -1013,7 +921,11 @@ cudaError_t launch_gather_ev(const double* ev, const int64_t* off_n, const int32
 
 cudaError_t launch_eigen_chain(const EigenBatch& E, cudaStream_t st) {
   if (E.count <= 0) return cudaSuccess;
-  eigen_chain_kernel<<<(E.count + 31) / 32, 32, 0, st>>>(E);
+  static std::atomic<uint64_t> raised{0};
+  cudaError_t e = raise_smem_limit_once((const void*)eigen_chain_kernel, raised);
+  if (e != cudaSuccess) return e;
+  const int stride = std::min(E.nmax, E.chain_nmax) | 1;
+  eigen_chain_kernel<<<(E.count + CH_M - 1) / CH_M, 32, sizeof(double) * CH_M * stride, st>>>(E);
   return cudaGetLastError();
 }
 

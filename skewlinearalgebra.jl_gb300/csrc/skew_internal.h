@@ -140,6 +140,7 @@ struct TrieigParams {
                            // then their indices and active sizes (solved by a second kernel)
   int grid;                // CTAs of the fallback kernel
   int max_iter = 0;        // QR sweeps before SKEW_NO_CONVERGENCE (0: 30 n, skeweigen.jl:115)
+  int nmax = 0;            // largest size (shared memory per matrix)
 };
 cudaError_t launch_batch_trieig(const TrieigParams& P, cudaStream_t st);
 

@@ -2,11 +2,8 @@
 //
 // Batched path: the implicit-QR iteration of skewtrieigvals!
 // (skeweigen.jl:105-156) with its exact tolerances, shift, deflation order and
-// stagnation rule, one matrix per thread.  The iteration is a serial chain of
-// Givens rotations; since the FP64 pipe charges a warp instruction the same
-// whether one lane or 32 are active, 32 matrices share each warp (matrices are
-// sorted by size, so warp-mates run similar trip counts).  A matrix whose
-// shifts stagnate is handed to a second kernel that solves the reference's
+// stagnation rule, four lanes per matrix (skew_chain.cuh; matrices are sorted by
+// size, so warp-mates run similar trip counts).  A matrix whose shifts stagnate is handed to a second kernel that solves the reference's
 // fallback, the eigenvalues of SymTridiagonal(0, ev) (skeweigen.jl:134-137,
 // 463-468), with one CTA per matrix and one eigenvalue per thread.
 //
@@ -20,8 +17,9 @@
 
 #include <algorithm>
 
-#include "skew_common.cuh"
 #include "skew_internal.h"
+#include "skew_chain.cuh"
+#include "skew_common.cuh"
 #include "skew_twisted.cuh"
 
 namespace skew {
@@ -68,50 +66,6 @@ __device__ void reducetozero_dev(double* ev, int n) {
   if (n == 2) ev[1] = __dadd_rn(__dmul_rn(s, a), __dmul_rn(b, c));
 }
 
-// implicitstep_novec (skeweigen.jl:73-103); n = active size - 1, start 1-based.
-// The chain is serial: step i needs the rotation of step i-1.  The three entries
-// a step reads besides ev[i+1] are the ones the previous step just wrote, so they
-// are carried in registers instead of going through memory, and ev[i+1], which no
-// step of this sweep has touched yet, is loaded one step ahead.  Every store of
-// the reference's step is still made, in the same order, so ev holds the same
-// values at every step and after an early return.
-__device__ int implicitstep_dev(double* ev, int n, int start) {
-  double bulge = 0.0;
-  const double shift = __dmul_rn(ev[n - 1], ev[n - 1]);
-  const double tol = 2.220446049250313e-16;  // eps(Float64)
-  double a = 0.0;              // ev[i-2] (zero at i == start, as the reference's alpha)
-  double b = ev[start - 1];    // ev[i-1]
-  double g = ev[start];        // ev[i]
-  double z = (start < n - 1) ? ev[start + 1] : 0.0;  // ev[i+1], untouched this sweep
-  for (int i = start; i <= n - 1; i++) {
-    const double zn = (i + 2 <= n - 1) ? ev[i + 2] : 0.0;  // next step's ev[i+1]
-    double c, s;
-    if (i > start) {
-      givens(a, bulge, c, s);
-    } else {
-      const double x1 = __dadd_rn(__dsub_rn(neg(__dmul_rn(a, a)), __dmul_rn(b, b)), shift);
-      const double x2 = __dadd_rn(neg(__dmul_rn(a, bulge)), __dmul_rn(b, g));
-      givens(x1, x2, c, s);
-    }
-    if (i > 1) ev[i - 2] = __dadd_rn(__dmul_rn(c, a), __dmul_rn(s, bulge));
-    const double nb = __dsub_rn(__dmul_rn(c, b), __dmul_rn(s, g));
-    const double ng = __dadd_rn(__dmul_rn(s, b), __dmul_rn(c, g));
-    ev[i - 1] = nb;
-    ev[i] = ng;
-    if (i < n - 1) {
-      const double nz = __dmul_rn(z, c);
-      ev[i + 1] = nz;
-      bulge = __dmul_rn(s, z);
-      if (fabs(bulge) < tol && fabs(nb) < tol) return i + 1;
-      a = nb;
-      b = ng;
-      g = nz;
-      z = zn;
-    }
-  }
-  return start;
-}
-
 // Number of eigenvalues of SymTridiagonal(0, e) (size n) smaller than x: the
 // count of negative pivots of the LDL^T factorisation of (T - x I), a pivot
 // smaller than pivmin in magnitude being replaced by -pivmin before it is
@@ -129,73 +83,40 @@ __device__ int sturm_count(const double* e, int n, double x, double pivmin) {
   return c;
 }
 
-// skewtrieigvals! (skeweigen.jl:105-156).  ev (N-1 entries) is destroyed;
-// vals[N] receives the imaginary parts in the reference's order.  On stagnation
-// the active size n is returned in *fb_n (vals[0..n) and ev[0..n-1) are then
-// left to the fallback kernel).
-__device__ int skewtrieigvals_dev(double* ev, int N, double* vals, int* fb_n, int max_iter_cap) {
-  int n = N;
-  for (int i = 0; i < N; i++) vals[i] = 0.0;
-  if (n & 1) {
-    n -= 1;
-    reducetozero_dev(ev, n);
+// skewtrieigvals! (skeweigen.jl:105-156), four lanes per matrix (skew_chain.cuh); vals
+// receives the imaginary parts in the reference's order.  On stagnation the matrix is left
+// to the fallback kernel: its active size, the values found so far and ev as it stands.
+__global__ void __launch_bounds__(32) batch_trieig_kernel(TrieigParams P) {
+  extern __shared__ double chain_ev[];
+  const int t = blockIdx.x * CH_M + threadIdx.x / CH_G, g = threadIdx.x & (CH_G - 1);
+  double* ev = chain_ev + (threadIdx.x / CH_G) * (P.nmax | 1);
+  Chain<false> S;
+  S.run = false;
+  S.status = SKEW_OK;
+  int b = 0, N = 0;
+  if (t < P.count) {
+    b = P.order[t];
+    N = P.n[b];
+    for (int i = g; i + 1 < N; i += CH_G) ev[i] = P.ev_all[P.ev_off[b] + i];
+    for (int i = g; i < N; i += CH_G) P.vals[b][i] = 0.0;
   }
-  const double tol = 10.0 * 2.220446049250313e-16;
-  const int max_iter = max_iter_cap > 0 ? max_iter_cap : 30 * n;
-  int iter = 0, count_static = 0, start = 1;
-  double mem = 1.0;
-  while (n > 2 && iter < max_iter) {
-    start = implicitstep_dev(ev, n - 1, start);
-    while (n > 2 && fabs(ev[n - 2]) <= tol) {
-      vals[n - 1] = 0.0;
-      n -= 1;
-    }
-    while (n > 2 && fabs(ev[n - 3]) <= tol * fabs(ev[n - 2])) {
-      vals[n - 2] = ev[n - 2];
-      vals[n - 1] = neg(ev[n - 2]);
-      n -= 2;
-    }
-    if (start > n - 2) start = 1;
-    if (n > 1 && fabs(mem - ev[n - 2]) < 0.0001 * fabs(ev[n - 2])) {
-      count_static += 1;
-      if (count_static > 4) {  // stagnation: symmetric tridiagonal fallback (:134-137)
-        *fb_n = n;
-        return SKEW_FALLBACK_USED;
-      }
-    } else {
-      count_static = 0;
-    }
-    mem = (n > 1 ? ev[n - 2] : 0.0);
-    iter += 1;
-  }
-  if (n == 2) {
-    vals[0] = ev[0];
-    vals[1] = neg(ev[0]);
-    return SKEW_OK;
-  }
-  if (n <= 1) {
-    if (n == 1) vals[0] = 0.0;
-    return SKEW_OK;
-  }
-  return SKEW_NO_CONVERGENCE;
-}
-
-__global__ void batch_trieig_kernel(TrieigParams P) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  __syncwarp();
+  if (N >= 1 && (N & 1) && g == 0) reducetozero_dev(ev, N - 1);
+  __syncwarp();
+  S.nb = S.bulge = S.q1 = S.q2 = S.shift = 0.0;
+  S.i = S.m = S.start = 0;
+  if (N >= 1) S.begin(ev, N & ~1, P.vals[b], P.max_iter, 1, nullptr, 0);
+  while (__any_sync(0xffffffffu, S.run)) S.step();
   if (t >= P.count) return;
-  const int b = P.order[t];
-  const int N = P.n[b];
-  double* ev = P.evwork + P.ev_off[b];
-  if (P.evwork != P.ev_all)
-    for (int i = 0; i + 1 < N; i++) ev[i] = P.ev_all[P.ev_off[b] + i];
-  int fb_n = 0;
-  const int st = (N >= 1) ? skewtrieigvals_dev(ev, N, P.vals[b], &fb_n, P.max_iter) : SKEW_OK;
-  if (st == SKEW_FALLBACK_USED) {
-    const unsigned k = atomicAdd(P.fallback, 1u);
-    P.fallback[2 + k] = (unsigned)b;
-    P.fallback[2 + P.count + k] = (unsigned)fb_n;
+  if (S.status == SKEW_FALLBACK_USED) {
+    for (int i = g; i + 1 < N; i += CH_G) P.evwork[P.ev_off[b] + i] = ev[i];
+    if (g == 0) {
+      const unsigned k = atomicAdd(P.fallback, 1u);
+      P.fallback[2 + k] = (unsigned)b;
+      P.fallback[2 + P.count + k] = (unsigned)S.fb_n;
+    }
   }
-  if (P.status) P.status[b] = st;
+  if (P.status && g == 0) P.status[b] = S.status;
 }
 
 constexpr int FB_NT = 256;
@@ -260,8 +181,10 @@ cudaError_t launch_batch_trieig(const TrieigParams& P, cudaStream_t st) {
   if (P.count <= 0) return cudaSuccess;
   cudaError_t e = cudaMemsetAsync(P.fallback, 0, 2 * sizeof(unsigned), st);
   if (e != cudaSuccess) return e;
-  const int bs = 32;
-  batch_trieig_kernel<<<(P.count + bs - 1) / bs, bs, 0, st>>>(P);
+  static std::atomic<uint64_t> raised{0};
+  e = raise_smem_limit_once((const void*)batch_trieig_kernel, raised);
+  if (e != cudaSuccess) return e;
+  batch_trieig_kernel<<<(P.count + CH_M - 1) / CH_M, 32, sizeof(double) * CH_M * (P.nmax | 1), st>>>(P);
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   batch_fallback_kernel<<<P.grid > 0 ? P.grid : 1, FB_NT, 0, st>>>(P);
