@@ -83,6 +83,11 @@ struct skew_batch_plan_st {
   double** e_p_work = nullptr;     // work + off_w per matrix
   int* e_status = nullptr;
   unsigned* e_counter = nullptr;
+  // gradients of log|Pf| on the tensor cores (global-memory buckets): allocated on first use
+  double* pg_ws = nullptr;
+  double* pg_tau = nullptr;
+  double** pg_refl = nullptr;  // [count] a matrix's workspace, null outside those buckets
+  int pg_state = 0;            // 0: not tried, 1: ready, -1: no memory (the fused kernel runs)
   int* e_exps = nullptr;  // exponents of the tiled products' operands (2 x ev_total)
   int* e_fsel = nullptr;  // exp adjoint: per matrix, real Schur-basis (1) or complex (0) form
   int32_t* e_back_off = nullptr;  // back-transformation items before each matrix (processing order)
@@ -651,7 +656,7 @@ int skew_batch_plan_destroy(skew_batch_plan_t P) {
   void* eig[] = {P->e_refl, P->e_tau, P->e_evb, P->e_G, P->e_log, P->e_work, P->e_vr, P->e_vi, P->e_vals,
                  P->e_off_log, P->e_cap_log, P->e_log_len, P->e_off_w, P->e_p_refl, P->e_p_vr, P->e_p_vi,
                  P->e_p_vals, P->e_p_scratch, P->e_p_work, P->e_status, P->e_fsel, P->e_exps, P->e_back_off,
-                 P->e_counter};
+                 P->e_counter, P->pg_ws, P->pg_tau, P->pg_refl};
   for (void* q : eig)
     if (q) cudaFreeAsync(q, st);
   if (P->fv_idx) cudaFreeAsync(P->fv_idx, st);
@@ -661,6 +666,41 @@ int skew_batch_plan_destroy(skew_batch_plan_t P) {
     if (q) cudaFreeAsync(q, st);
   cudaStreamSynchronize(st);
   delete P;
+  return SKEW_OK;
+}
+
+// Workspace of the tensor-core gradients.  Without the memory for it the plan keeps the
+// fused kernel, which needs none.
+static int pfgrad_ws(skew_batch_plan_t P) {
+  if (P->pg_state != 0) return SKEW_OK;
+  P->pg_state = -1;
+  cudaStream_t st = P->h->stream;
+  std::vector<int32_t> order(P->count);
+  std::iota(order.begin(), order.end(), 0);
+  std::stable_sort(order.begin(), order.end(), [&](int32_t a, int32_t c) { return P->n_host[a] > P->n_host[c]; });
+  std::vector<size_t> off(P->count, SIZE_MAX);
+  size_t total = 0;
+  for (const Bucket& B : P->buckets) {
+    if (B.smem_matrix) continue;
+    for (int t = B.begin; t < B.end; t++) {
+      off[order[t]] = total;
+      total += pfgrad_ws_doubles(P->n_host[order[t]]);
+    }
+  }
+  if (total == 0) return SKEW_OK;
+  if (cudaMallocAsync(&P->pg_ws, sizeof(double) * total, st) != cudaSuccess) {
+    (void)cudaGetLastError();
+    P->pg_ws = nullptr;
+    return SKEW_OK;
+  }
+  CK(cudaMallocAsync(&P->pg_tau, sizeof(double) * P->ev_total, st));
+  CK(cudaMallocAsync(&P->pg_refl, sizeof(double*) * P->count, st));
+  std::vector<double*> ptr(P->count, nullptr);
+  for (int64_t b = 0; b < P->count; b++)
+    if (off[b] != SIZE_MAX) ptr[b] = P->pg_ws + off[b];
+  CK(cudaMemcpyAsync(P->pg_refl, ptr.data(), sizeof(double*) * P->count, cudaMemcpyHostToDevice, st));
+  CK(cudaStreamSynchronize(st));  // ptr goes out of scope
+  P->pg_state = 1;
   return SKEW_OK;
 }
 
@@ -696,7 +736,28 @@ static int run_buckets(skew_batch_plan_t P, const double* const* A, double* logp
     bp.status = status;
     bp.host_in = host_in ? 1 : 0;
     bp.grad_host = grad_host;
+    // gradients of the global-memory matrices: the reduction alone, then the products of all
+    // of them on the tensor cores
+    const bool pg = grad && !B.smem_matrix && !host_in && !grad_host && P->pg_state == 1;
+    if (pg) {
+      bp.grad = nullptr;
+      bp.ev_out = P->d_ev;
+      bp.tau_out = P->pg_tau;
+      bp.refl_out = P->pg_refl;
+    }
     CK(launch_batch_pf(bp, B.grid, st, tridiag_only));
+    if (pg) {
+      PfGrad g;
+      g.order = P->d_order + B.begin;
+      g.n = P->d_n;
+      g.off = P->d_ev_off;
+      g.ev = P->d_ev;
+      g.tau = P->pg_tau;
+      g.refl = P->pg_refl;
+      g.grad = grad;
+      g.status = status;
+      CK(launch_pfgrad(g, B.end - B.begin, B.nmax, st));
+    }
   }
   return SKEW_OK;
 }
@@ -772,6 +833,10 @@ int skew_batch_logabspf_d(skew_batch_plan_t P, const double* const* A, double* l
                           double* const* grad, int* status) {
   if (!P || (P->count > 0 && (!A || !logpf || !sign || !status))) return SKEW_BAD_ARG;
   if (P->count == 0) return SKEW_OK;
+  if (grad) {
+    const int s = pfgrad_ws(P);
+    if (s) return s;
+  }
   return graph_issue(P, G_LOGPF, {A, logpf, sign, grad, status, nullptr},
                      [&] { return run_buckets(P, A, logpf, sign, grad, status, false); });
 }

@@ -41,6 +41,7 @@ struct BackTask {
   int nc[2];
   double *t, *vt, *w;     // T: panels of ldt x ldt; VT: R n x nref; W: R ldt x columns (x splits)
   int *et, *evt, *ex;     // exponents: T's columns, VT's rows per panel, X's columns
+  int identity;           // X starts as the identity: a panel from column c0 leaves columns 0 .. c0 alone
   int* status;
   __host__ __device__ int ldt() const { return nref < BK<CX>::PB ? nref : BK<CX>::PB; }
   __host__ __device__ int panels() const { return (nref + BK<CX>::PB - 1) / BK<CX>::PB; }
@@ -372,6 +373,7 @@ __global__ void __launch_bounds__(OZ_NT, 1) back_w_kernel(Src S, int step) {
   const int p = P.B.panels() - 1 - step;
   if (p < 0 || (int)blockIdx.x * OZ_N >= P.B.cols()) return;
   const int c0 = p * BK<CX>::PB, nb = min(BK<CX>::PB, P.B.nref - c0);
+  if (P.B.identity && (int)blockIdx.x * OZ_N + OZ_N - 1 <= c0) return;
   P.V = BackV<CX, true>{P.B.A, P.B.tau, P.B.lda, c0, nb, P.B.n};
   const int all = (BK<CX>::R * (P.B.n - c0 - 1) + OZ_K - 1) / OZ_K;
   const int chunks = (all + 3) / 4, per = (chunks + gridDim.y - 1) / gridDim.y * 4;  // whole exact sums
@@ -403,7 +405,7 @@ __global__ void __launch_bounds__(OZ_NT, 1) back_x_kernel(Src S, int step, int r
   P.c0 = P.p * BK<CX>::PB;
   P.nb = min(BK<CX>::PB, P.B.nref - P.c0);
   const int i0 = (int)(blockIdx.x % rt) * OZ_M, j0 = (int)(blockIdx.x / rt) * OZ_N;
-  if (i0 >= P.rows() || j0 >= P.cols()) return;
+  if (i0 >= P.rows() || j0 >= P.cols() || (P.B.identity && j0 + OZ_N - 1 <= P.c0)) return;
   oz_tile(P, i0, j0, oz_buf);
 }
 

@@ -718,6 +718,7 @@ cudaError_t zeigen_from_tridiag(const double* Ad, int64_t lda, int n, const doub
   S.B.ldx = ldv;
   S.B.nc[0] = n;
   S.B.nc[1] = 0;
+  S.B.identity = 0;
   S.B.status = nullptr;
   int splits = 1;
   if (nextra) {

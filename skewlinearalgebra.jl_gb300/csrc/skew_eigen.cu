@@ -896,6 +896,7 @@ struct BatchBack {
     T.nc[0] = n;
     T.nc[1] = qonly ? 0 : n;
     T.ldx = n;
+    T.identity = 0;
     T.status = E.status + b;
     const size_t nn = (size_t)n * n;
     back_ws_set(T, E.pwork[b] + (batch_back_doubles(n) <= 2 * nn ? nn : (size_t)max((int64_t)(4 * nn), fallback_ws_doubles(n))), 2 * n, 1);

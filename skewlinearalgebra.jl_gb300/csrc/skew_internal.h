@@ -301,6 +301,21 @@ cudaError_t launch_eigen_func(const EigenBatch& E, int mode, cudaStream_t st);
 // exp adjoint: the real Schur basis Q (and fsel) from vals, Vr, Vi into pwork
 cudaError_t launch_schur_basis(const EigenBatch& E, cudaStream_t st);
 
+// Gradients of log|Pf| of the matrices order[0 .. count) of a batch (largest first) from
+// their reduction, on the tensor cores (skew_pfgrad.cu).
+struct PfGrad {
+  const int32_t* order;
+  const int32_t* n;
+  const int64_t* off;     // packed offsets of ev and tau
+  const double* ev;
+  const double* tau;
+  double* const* refl;    // per matrix: pfgrad_ws_doubles(n), the reflectors first
+  double* const* grad;
+  int* status;            // SKEW_OK: the gradient exists (else NaN)
+};
+size_t pfgrad_ws_doubles(int n);
+cudaError_t launch_pfgrad(const PfGrad& P, int count, int nmax, cudaStream_t st);
+
 // One real matrix with n > kWideMin (skew_wide.cu): the product of the panel in fixed point,
 // the trailing update on the tensor cores.  cudaErrorNotSupported (nothing done) where it
 // cannot run; the caller then takes the kernels below.

@@ -614,6 +614,7 @@ static cudaError_t back_transform(const double* A, int64_t lda, const double* ta
   S.B.ldx = ldv;
   S.B.nc[0] = n - cr0;
   S.B.nc[1] = n - ci0;
+  S.B.identity = 0;
   S.B.status = nullptr;
   S.gate = L.gate;
   S.gate_on = L.gate_on;
