@@ -219,17 +219,17 @@ def logabspfaffian_(A, check_skew: bool = False) -> Tuple[float, float]:
     """logabspfaffian!(A): in place, returns (log|Pf(A)|, sign)."""
     S = _as_skew(A) if not isinstance(A, torch.Tensor) else SkewHermitian(A, check_skew=False)
     n = S.n
-    out = torch.zeros(2, dtype=torch.float64, device="cuda")
-    info = _info_tensor()
+    # log|Pf|, sign and info (int32) in one buffer that the call fills: one copy to the host
+    out = torch.empty(3, dtype=torch.float64, device="cuda")
+    p = out.data_ptr()
     h = handle().bind()
-    check(_lib.load().skew_logabspf_d(h, _ptr(S.data), n, n, ctypes.c_void_p(out.data_ptr()),
-                                      ctypes.c_void_p(out.data_ptr() + 8), int(check_skew), _ptr(info)),
+    check(_lib.load().skew_logabspf_d(h, _ptr(S.data), n, n, ctypes.c_void_p(p), ctypes.c_void_p(p + 8),
+                                      int(check_skew), ctypes.c_void_p(p + 16)),
           "logabspfaffian")
-    st = int(info.item())
-    if st == _lib.SKEW_NOT_SKEW:
+    host = out.cpu().numpy()
+    if int(host[2:].view(np.int32)[0]) == _lib.SKEW_NOT_SKEW:
         raise ValueError("Pfaffian requires a skew-Hermitian matrix")
-    lp, sg = out.tolist()
-    return lp, sg
+    return float(host[0]), float(host[1])
 
 
 def _is_complex(A) -> bool:
