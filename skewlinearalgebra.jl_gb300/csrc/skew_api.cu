@@ -293,6 +293,11 @@ int skew_set_stream(skew_handle_t h, skew_stream_t s) {
 // which single-matrix calls use the multi-CTA blocked reduction instead (the
 // tuning key blocked_min_n).
 static const int64_t kSingleMax = 1024;
+// Functions of one matrix above this size take the whole GPU (func_large); their result
+// does not depend on the eigenvalues' order.  exp as a batch of one (one CTA reduces the
+// matrix) against the whole GPU: n = 64 0.96 / 1.07 ms, 96 1.63 / 1.57, 128 2.23 / 1.95,
+// 256 7.9 / 3.7, 512 45.4 / 8.6, 1000 302 / 24.4.
+static const int64_t kFuncLargeMin = 95;
 static int64_t blocked_min_n(skew_handle_t h) { return h->tune.blocked_min_n; }
 
 static int single(skew_handle_t h, double* A, int64_t n, int64_t lda, double* G, int64_t ldg, double* logpf,
@@ -321,8 +326,10 @@ static size_t reduce_ws_doubles(int64_t n) {
 }
 
 // Blocked reduction of a large matrix into tau/ev (device); A in place.
+// qr_order: the caller runs the QR chain on ev up to n = 1024, whose deflation order
+// depends on the last bits, so the reduction keeps its arithmetic there.
 static int blocked(skew_handle_t h, double* A, int64_t n, int64_t lda, double* tau, double* ev, int* info,
-                   size_t extra_doubles, double** extra) {
+                   size_t extra_doubles, double** extra, bool qr_order = false) {
   if (!h || !A || lda < n || n > (1LL << 15)) return n > (1LL << 15) ? SKEW_UNSUPPORTED : SKEW_BAD_ARG;
   const size_t wsd = reduce_ws_doubles(n);
   int st = ensure_ws(h, sizeof(double) * (wsd + extra_doubles));
@@ -343,9 +350,8 @@ static int blocked(skew_handle_t h, double* A, int64_t n, int64_t lda, double* t
     if (e != cudaErrorNotSupported) return SKEW_CUDA_ERROR;
     cudaGetLastError();
   }
-  // above kWideMin: the panel's product in fixed point, the trailing update on the
-  // tensor cores
-  if (n > kWideMin && h->tune.blocked_persistent != 0) {
+  // the panel's product in fixed point, the trailing update on the tensor cores
+  if (n > (qr_order ? kSingleMax : kWideMin) && h->tune.blocked_persistent != 0) {
     cudaError_t e = wide_hessenberg(A, lda, (int)n, tau, ev, info, ws, h->sms, h->tune, h->stream);
     if (e == cudaSuccess) return SKEW_OK;
     if (e != cudaErrorNotSupported && e != cudaErrorCooperativeLaunchTooLarge) return SKEW_CUDA_ERROR;
@@ -443,7 +449,7 @@ int skew_eigvals_d(skew_handle_t h, double* A, int64_t n, int64_t lda, double* v
   double* ev = nullptr;
   if (n >= blocked_min_n(h)) {
     double* extra = nullptr;
-    st = blocked(h, A, n, lda, nullptr, nullptr, info, 2 * (size_t)n + 2, &extra);
+    st = blocked(h, A, n, lda, nullptr, nullptr, info, 2 * (size_t)n + 2, &extra, true);
     if (st) return st;
     ev = extra;
   } else {
@@ -1311,10 +1317,8 @@ static int single_func(skew_handle_t h, double* A, int64_t n, int64_t lda, doubl
                        int func = SKEW_FUNC_EXP) {
   if (!h || n < 1 || !A || lda != n || (ldv && ldv != n) || (ldo && ldo != n)) return n < 1 ? SKEW_BAD_ARG
                                                                                             : SKEW_UNSUPPORTED;
-  if (n > kSingleMax) {
-    if (mode < 0) return SKEW_UNSUPPORTED;  // eigen of large matrices: eigen_large
-    return func_large(h, A, nullptr, n, out, cot, mode, func, info);
-  }
+  if (n > kSingleMax && mode < 0) return SKEW_UNSUPPORTED;  // eigen of large matrices: eigen_large
+  if (mode >= 0 && n > kFuncLargeMin) return func_large(h, A, nullptr, n, out, cot, mode, func, info);
   skew_batch_plan_t P = nullptr;
   int s = single_plan(h, n, &P);
   if (s) return s;

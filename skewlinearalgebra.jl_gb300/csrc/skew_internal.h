@@ -318,8 +318,9 @@ cudaError_t launch_pfgrad(const PfGrad& P, int count, int nmax, cudaStream_t st)
 
 // One real matrix with n > kWideMin (skew_wide.cu): the product of the panel in fixed point,
 // the trailing update on the tensor cores.  cudaErrorNotSupported (nothing done) where it
-// cannot run; the caller then takes the kernels below.
-constexpr int kWideMin = 1024;
+// cannot run; the caller then takes the kernels below.  Up to kWideMin the cluster reduction
+// is faster (n = 600: 7.3 ms; 650 here 10.6, the grid-wide kernel 11.3).
+constexpr int kWideMin = 640;
 size_t wide_ws_doubles(int n);
 cudaError_t wide_hessenberg(double* A, int64_t lda, int n, double* tau, double* ev, int* info, double* ws, int sms,
                             const Tuning& T, cudaStream_t st);

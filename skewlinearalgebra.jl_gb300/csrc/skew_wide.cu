@@ -1,4 +1,4 @@
-// Blocked Householder tridiagonalisation of one real skew matrix with n > 1024 (the
+// Blocked Householder tridiagonalisation of one real skew matrix with n > 640 (the
 // skewblockedhess! / skewlatrd! structure of hessenberg.jl:92-173), with the two O(n^3)
 // parts off the FP64 pipe.
 //
@@ -17,8 +17,8 @@
 // Whole reduction: n = 1025 19.0 -> 17.4 ms, 2048 51.0 -> 37.6, 4096 195 -> 96, 8192 929 -> 366
 // (panels 305, update 52, packing 5).
 //
-// n <= 1024 keeps the kernels of skew_blocked.cu and skew_cluster.cu: the reference-order
-// eigenvalues of those sizes depend on the last bits of the tridiagonal.
+// Eigenvalues in the QR's deflation order (n <= 1024) keep the kernels of skew_blocked.cu
+// and skew_cluster.cu: the order depends on the last bits of the tridiagonal.
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>

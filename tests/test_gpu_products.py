@@ -97,3 +97,23 @@ def test_not_finite_cotangent_gives_nan(bad):
     assert np.isnan(G0).all()
     want = _frechet(mats[1], cots[1])
     assert np.linalg.norm(G1 - want) <= 40 * 70 * EPS * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("n", [95, 96, 97, 160, 333, 640, 641, 700, 1024])
+def test_single_matrix_functions_at_the_dispatch_edges(n):
+    """exp and its adjoint of one matrix around the sizes where the whole GPU takes over (96) and
+    where its reduction changes (641)."""
+    import scipy.linalg as sl
+    import skewgpu
+
+    (A,), rng = _batch([n], 10 + n)
+    want = sl.expm(A)
+    assert np.linalg.norm(skewgpu.exp(A) - want) <= 40 * n * EPS * np.linalg.norm(want)
+    if n <= 333:
+        C = rng.standard_normal((n, n))
+        _, pullback = skewgpu.exp_rrule(A)
+        ref = _frechet(A, C)
+        assert np.linalg.norm(pullback(C) - ref) <= 40 * n * EPS * np.linalg.norm(ref)
+    if n % 2:
+        with pytest.raises(ValueError):
+            skewgpu.matrix_function(A, "log")
