@@ -271,9 +271,10 @@ struct EigenBatch {
 // bisection (values descending, exact +-pairs, also into vals_out[idx[mb]]) and
 // twisted-factorisation vectors with the banded orthogonal correction, written in
 // the tridiagonal basis to Vr[idx[mb]], Vi[idx[mb]] (n x n, leading dimension n).
-// ws: G x skew_vectors_batch_ws_doubles(n); bp_g: 8 G; vals_g: n G.
+// ws: G x skew_vectors_batch_ws_doubles(n); bp_g: 8 G; vals_g: n G.  beside: how many
+// launches like this one share the GPU.
 cudaError_t launch_tridiag_bisect_batch(const double* e_g, int n, int G, double* bp_g, double* vals_g,
-                                        double* const* vals_out, const int32_t* idx, cudaStream_t st);
+                                        double* const* vals_out, const int32_t* idx, int beside, cudaStream_t st);
 size_t skew_vectors_batch_ws_doubles(int n);
 cudaError_t skew_vectors_batch(const double* e_g, int n, int G, const double* vals_g, const double* bp_g,
                                double* const* Vr, double* const* Vi, const int32_t* idx, double* ws,

@@ -340,7 +340,7 @@ __global__ void bisect_batch_kernel(const double* __restrict__ e_g, int n, const
 }
 
 cudaError_t launch_tridiag_bisect_batch(const double* e_g, int n, int G, double* bp_g, double* vals_g,
-                                        double* const* vals_out, const int32_t* idx, cudaStream_t st) {
+                                        double* const* vals_out, const int32_t* idx, int beside, cudaStream_t st) {
   if (n <= 0 || G <= 0) return cudaSuccess;
   bisect_prep_batch_kernel<<<G, 256, 0, st>>>(e_g, n, bp_g);
   cudaError_t e = cudaGetLastError();
@@ -349,7 +349,7 @@ cudaError_t launch_tridiag_bisect_batch(const double* e_g, int n, int G, double*
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int h = n / 2;
   // lanes per eigenvalue: the whole batch shares the machine
-  const int p = multisect_lanes(std::max(1, h * G), sms);
+  const int p = multisect_lanes(std::max(1, h * G * beside), sms);
   const long long threads = ((long long)std::max(h, 1) * p + 31) / 32 * 32;
   const int bs = 128;
   const size_t smem = n <= STURM_STAGE ? n * sizeof(double) : 0;
