@@ -1530,21 +1530,15 @@ static int zreduce(skew_handle_t h, double* A, int64_t n, int64_t lda, int64_t B
                    double* dvim, double* zws, int* info = nullptr) {
   if (B > 1 || n <= 128) {
     ZHessParams P;
-    P.W = nullptr;
-    P.W1 = A;
-    P.n1 = (int)n;
-    P.ld1 = lda;
+    P.W = A;
     P.stride = lda * n;
-    P.n = nullptr;
-    P.order = nullptr;
-    P.off = nullptr;
+    P.ld = lda;
+    P.n = (int)n;
     P.count = (int32_t)B;
-    P.nmax = (int)n;
-    P.counter = nullptr;
     P.tau = tau;
     P.ev = ev;
     P.dvim = dvim;
-    CK(launch_zhess_cta(P, (int)B, h->stream));
+    CK(launch_zhess_cta(P, h->stream));
     return SKEW_OK;
   }
   if (n >= zpersist_min_n(h)) {

@@ -20,6 +20,7 @@
 // large reduction); and per-column multi-CTA kernels for large n (reflector,
 // matvec partials over (row block, column chunk) tiles, combination, and the
 // rank-2 update on 32 x 32 tiles of the lower triangle with a transposed mirror).
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
@@ -33,6 +34,8 @@
 #include "skew_funcs.cuh"
 
 namespace skew {
+
+namespace cg = cooperative_groups;
 
 constexpr int ZNT = 256;
 constexpr int ZNW = ZNT / 32;
@@ -62,7 +65,7 @@ __device__ ZRefl zrefl(zc alpha, double xnorm) {
 }
 
 // ---------------------------------------------------------------------------
-// one CTA per matrix
+// one cluster of CTAs per matrix
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ double block_max(double x, double* red) {
 #pragma unroll
@@ -77,156 +80,222 @@ __device__ __forceinline__ double block_max(double x, double* red) {
   return s;
 }
 
+// One cluster of CS CTAs per matrix, P.count matrices.  Bound by the FP64 pipe (8/3 n^3 complex
+// multiply-adds' worth of FMAs per matrix), so the cluster is as wide as fills the SMs: the
+// CTAs share the rows of A22 v (interleaved blocks of 32 rows, a block's columns split over
+// the warps that have no block) and the entries of the update, exchange W through
+// distributed shared memory and each form the reflector themselves.  The matrix lies in
+// global memory (L2); what another CTA wrote is read with L2-only loads.
+// 64 x n = 256: 20.4 -> 13.3 ms (clusters of 4; one CTA per matrix before).
+template <int CS>
 __global__ void __launch_bounds__(ZNT) zhess_cta_kernel(ZHessParams P) {
-  extern __shared__ __align__(16) double zsm[];  // v (nmax complex) | w (nmax complex)
+  extern __shared__ __align__(16) double zsm[];  // x, then v (n complex) | w (n complex)
+  const int n = P.n;
   zc* vs = reinterpret_cast<zc*>(zsm);
-  zc* ws = vs + P.nmax;
+  zc* ws = vs + n;
   __shared__ double red[ZNW];
-  __shared__ int s_next;
+  __shared__ zc part[ZNT];
   __shared__ ZRefl s_R;
-  for (;;) {
-    if (threadIdx.x == 0) s_next = P.counter ? (int)atomicAdd(P.counter, 1u) : (int)blockIdx.x;
-    __syncthreads();
-    const int t = s_next;
-    __syncthreads();
-    if (t >= P.count) break;
-    const int b = P.order ? P.order[t] : t;
-    const bool one = (P.W == nullptr);  // matrices given directly: W1 + b * stride
-    const int n = one ? P.n1 : P.n[b];
-    const int64_t ld = one ? P.ld1 : n;
-    const int64_t off = one ? (int64_t)b * P.n1 : P.off[b];
-    zc* W = one ? reinterpret_cast<zc*>(P.W1) + (int64_t)b * P.stride : reinterpret_cast<zc*>(P.W[b]);
-    zc* tau = reinterpret_cast<zc*>(P.tau) + off;
-    double* ev = P.ev + off;
-    for (int c = 0; c + 1 < n; c++) {
-      const int m = n - c - 1;
-      zc* x = W + (c + 1) + (int64_t)c * ld;
-      double amax = 0.0;
-      for (int i = 1 + threadIdx.x; i < m; i += ZNT) amax = fmax(amax, fmax(fabs(x[i].re), fabs(x[i].im)));
-      amax = block_max(amax, red);
-      double ss = 0.0;
-      if (amax > 0.0) {
-        const double inv = 1.0 / amax;
-        for (int i = 1 + threadIdx.x; i < m; i += ZNT) {
-          const double a = x[i].re * inv, bb = x[i].im * inv;
+  cg::cluster_group cl = cg::this_cluster();
+  const int rank = CS > 1 ? (int)cl.block_rank() : 0;
+  const int b = blockIdx.x / CS;
+  const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
+  auto sync = [&]() {
+    if (CS > 1)
+      cl.sync();
+    else
+      __syncthreads();
+  };
+  auto ld2 = [](const zc* p) {
+    const double2 v = __ldcg(reinterpret_cast<const double2*>(p));
+    return zc{v.x, v.y};
+  };
+  const int64_t ld = P.ld;
+  zc* W = reinterpret_cast<zc*>(P.W) + (int64_t)b * P.stride;
+  zc* tau = reinterpret_cast<zc*>(P.tau) + (int64_t)b * n;
+  double* ev = P.ev + (int64_t)b * n;
+  for (int c = 0; c + 1 < n; c++) {
+    const int m = n - c - 1;
+    zc* x = W + (c + 1) + (int64_t)c * ld;
+    double amax = 0.0;
+    for (int i = tid; i < m; i += ZNT) {
+      const zc v = ld2(x + i);
+      vs[i] = v;
+      if (i > 0) amax = fmax(amax, fmax(fabs(v.re), fabs(v.im)));
+    }
+    amax = block_max(amax, red);
+    double ss = 0.0;
+    if (amax > 0.0) {
+      const double inv = 1.0 / amax;
+      for (int i = tid; i < m; i += ZNT)
+        if (i > 0) {
+          const double a = vs[i].re * inv, bb = vs[i].im * inv;
           ss = fma(a, a, fma(bb, bb, ss));
         }
-      }
-      ss = block_sum<ZNW>(ss, red);
-      if (threadIdx.x == 0) {
-        s_R = zrefl(x[0], amax * sqrt(ss));
+    }
+    ss = block_sum<ZNW>(ss, red);
+    if (tid == 0) {
+      s_R = zrefl(vs[0], amax * sqrt(ss));
+      if (rank == 0) {
         ev[c] = s_R.beta;
         tau[c] = s_R.tau;
       }
-      __syncthreads();
-      const ZRefl R = s_R;
-      const bool zero = (R.tau.re == 0.0 && R.tau.im == 0.0);
-      for (int i = threadIdx.x; i < m; i += ZNT) {
-        const zc v = zero ? zc{0.0, 0.0} : (i == 0 ? zc{1.0, 0.0} : zmul(x[i], R.scale));
-        x[i] = v;
-        vs[i] = v;
-      }
-      __syncthreads();
-      if (zero) continue;  // H = I: nothing to update
-      zc* A22 = W + (c + 1) + (int64_t)(c + 1) * ld;
-      // p = A22 v  (rows by threads, coalesced down each column; eight loads in
-      // flight per thread: the working copy of a batch lives in L2)
-      for (int i = threadIdx.x; i < m; i += ZNT) {
-        zc a0{0.0, 0.0}, a1{0.0, 0.0}, a2{0.0, 0.0}, a3{0.0, 0.0};
-        const zc* row = A22 + i;
-        int j = 0;
-        for (; j + 7 < m; j += 8) {
-          zc x[8];
-#pragma unroll
-          for (int u = 0; u < 8; u++) x[u] = row[(int64_t)(j + u) * ld];
-          a0 = zfma(x[0], vs[j], a0);
-          a1 = zfma(x[1], vs[j + 1], a1);
-          a2 = zfma(x[2], vs[j + 2], a2);
-          a3 = zfma(x[3], vs[j + 3], a3);
-          a0 = zfma(x[4], vs[j + 4], a0);
-          a1 = zfma(x[5], vs[j + 5], a1);
-          a2 = zfma(x[6], vs[j + 6], a2);
-          a3 = zfma(x[7], vs[j + 7], a3);
-        }
-        for (; j < m; j++) a0 = zfma(row[(int64_t)j * ld], vs[j], a0);
-        ws[i] = zmul(R.tau, zadd(zadd(a0, a1), zadd(a2, a3)));  // W = tau p
-      }
-      __syncthreads();
-      // a = tau (W^H v) / 2
-      double dr = 0.0, di = 0.0;
-      for (int i = threadIdx.x; i < m; i += ZNT) {
-        const zc d = zcmul(ws[i], vs[i]);  // conj(W_i) v_i
-        dr += d.re;
-        di += d.im;
-      }
-      dr = block_sum<ZNW>(dr, red);
-      di = block_sum<ZNW>(di, red);
-      const zc a = zmul(R.tau, zc{0.5 * dr, 0.5 * di});
-      for (int i = threadIdx.x; i < m; i += ZNT) ws[i] = zfma(a, vs[i], ws[i]);
-      __syncthreads();
-      // A22 += v w^H - w v^H on the lower triangle (diagonal included), mirrored.
-      // The triangle is walked column by column as one list of m (m + 1) / 2 entries
-      // (no division per entry); four entries per thread and iteration, loads first.
-      {
-        int j = 0, r = threadIdx.x;  // entry (j + r, j): column j has m - j entries
-        while (j < m && r >= m - j) {
-          r -= m - j;
-          j++;
-        }
-        while (j < m) {
-          int jj[4], ii[4];
-#pragma unroll
-          for (int u = 0; u < 4; u++) {
-            jj[u] = j;
-            ii[u] = j + r;
-            if (j < m) {
-              r += ZNT;
-              while (j < m && r >= m - j) {
-                r -= m - j;
-                j++;
-              }
-            }
-          }
-          zc a[4];
-#pragma unroll
-          for (int u = 0; u < 4; u++)
-            if (jj[u] < m) a[u] = A22[ii[u] + (int64_t)jj[u] * ld];
-#pragma unroll
-          for (int u = 0; u < 4; u++) {
-            if (jj[u] >= m) continue;
-            const int i = ii[u], jc = jj[u];
-            const zc vi = vs[i], wi = ws[i];
-            if (i == jc) {
-              a[u].im += 2.0 * (vi.im * wi.re - vi.re * wi.im);  // 2 Im(v conj(w))
-              A22[i + (int64_t)i * ld] = a[u];
-            } else {
-              const zc vj = vs[jc], wj = ws[jc];
-              const zc uu = zsub(zadd(a[u], zmulc(vi, wj)), zmulc(wi, vj));  // + v_i conj(w_j) - w_i conj(v_j)
-              A22[i + (int64_t)jc * ld] = uu;
-              A22[jc + (int64_t)i * ld] = zc{neg(uu.re), uu.im};  // -conj(u)
-            }
-          }
-        }
-      }
-      __syncthreads();
-    }
-    if (P.dvim) {
-      double* dv = P.dvim + off;
-      for (int k = threadIdx.x; k < n; k += ZNT) dv[k] = W[k + (int64_t)k * ld].im;
     }
     __syncthreads();
-    if (!P.counter) break;
+    const ZRefl R = s_R;
+    const bool zero = (R.tau.re == 0.0 && R.tau.im == 0.0);
+    for (int i = tid; i < m; i += ZNT)
+      vs[i] = zero ? zc{0.0, 0.0} : (i == 0 ? zc{1.0, 0.0} : zmul(vs[i], R.scale));
+    if (zero) {  // H = I: nothing to update
+      sync();    // every CTA has read x
+      for (int i = rank * ZNT + tid; i < m; i += ZNT * CS) x[i] = zc{0.0, 0.0};
+      continue;
+    }
+    __syncthreads();
+    zc* A22 = W + (c + 1) + (int64_t)(c + 1) * ld;
+    // W = tau A22 v: this CTA's row blocks rank, rank + CS, ...; eight loads in flight per thread
+    {
+      const int nb = (m + 31) / 32, mine = (nb - rank + CS - 1) / CS;
+      const int segs = mine > 0 ? max(1, ZNW / mine) : 1;
+      for (int q0 = 0; q0 < mine; q0 += ZNW) {
+        const int blocks = min(mine - q0, ZNW);
+        const int q = w % blocks, seg = w / blocks;
+        const int i = ((q0 + q) * CS + rank) * 32 + lane;
+        zc p{0.0, 0.0};
+        if (seg < segs && i < m) {
+          const int j1 = m * (seg + 1) / segs;
+          int j = m * seg / segs;
+          zc a0{0.0, 0.0}, a1{0.0, 0.0}, a2{0.0, 0.0}, a3{0.0, 0.0};
+          const zc* row = A22 + i;
+          for (; j + 7 < j1; j += 8) {
+            zc y[8];
+#pragma unroll
+            for (int u = 0; u < 8; u++) y[u] = ld2(row + (int64_t)(j + u) * ld);
+            a0 = zfma(y[0], vs[j], a0);
+            a1 = zfma(y[1], vs[j + 1], a1);
+            a2 = zfma(y[2], vs[j + 2], a2);
+            a3 = zfma(y[3], vs[j + 3], a3);
+            a0 = zfma(y[4], vs[j + 4], a0);
+            a1 = zfma(y[5], vs[j + 5], a1);
+            a2 = zfma(y[6], vs[j + 6], a2);
+            a3 = zfma(y[7], vs[j + 7], a3);
+          }
+          for (; j < j1; j++) a0 = zfma(ld2(row + (int64_t)j * ld), vs[j], a0);
+          p = zadd(zadd(a0, a1), zadd(a2, a3));
+        }
+        part[tid] = p;
+        __syncthreads();
+        if (w < blocks && i < m) {  // seg 0 joins the block's segments
+          for (int g = 1; g < segs; g++) p = zadd(p, part[(g * blocks + w) * 32 + lane]);
+          p = zmul(R.tau, p);
+          if (CS > 1) {
+#pragma unroll
+            for (int r = 0; r < CS; r++) cl.map_shared_rank(ws, r)[i] = p;
+          } else {
+            ws[i] = p;
+          }
+        }
+        __syncthreads();
+      }
+    }
+    sync();
+    for (int i = rank * ZNT + tid; i < m; i += ZNT * CS) x[i] = vs[i];
+    // a = tau (W^H v) / 2
+    double dr = 0.0, di = 0.0;
+    for (int i = tid; i < m; i += ZNT) {
+      const zc d = zcmul(ws[i], vs[i]);  // conj(W_i) v_i
+      dr += d.re;
+      di += d.im;
+    }
+    dr = block_sum<ZNW>(dr, red);
+    di = block_sum<ZNW>(di, red);
+    const zc a = zmul(R.tau, zc{0.5 * dr, 0.5 * di});
+    for (int i = tid; i < m; i += ZNT) ws[i] = zfma(a, vs[i], ws[i]);
+    __syncthreads();
+    // A22 += v w^H - w v^H on the lower triangle (diagonal included), mirrored.
+    // The triangle is walked column by column as one list of m (m + 1) / 2 entries
+    // (no division per entry); four entries per thread and iteration, loads first.
+    {
+      int j = 0, r = rank * ZNT + tid;  // entry (j + r, j): column j has m - j entries
+      while (j < m && r >= m - j) {
+        r -= m - j;
+        j++;
+      }
+      while (j < m) {
+        int jj[4], ii[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+          jj[u] = j;
+          ii[u] = j + r;
+          if (j < m) {
+            r += ZNT * CS;
+            while (j < m && r >= m - j) {
+              r -= m - j;
+              j++;
+            }
+          }
+        }
+        zc y[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+          if (jj[u] < m) y[u] = ld2(A22 + ii[u] + (int64_t)jj[u] * ld);
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+          if (jj[u] >= m) continue;
+          const int i = ii[u], jc = jj[u];
+          const zc vi = vs[i], wi = ws[i];
+          if (i == jc) {
+            y[u].im += 2.0 * (vi.im * wi.re - vi.re * wi.im);  // 2 Im(v conj(w))
+            A22[i + (int64_t)i * ld] = y[u];
+          } else {
+            const zc vj = vs[jc], wj = ws[jc];
+            const zc uu = zsub(zadd(y[u], zmulc(vi, wj)), zmulc(wi, vj));  // + v_i conj(w_j) - w_i conj(v_j)
+            A22[i + (int64_t)jc * ld] = uu;
+            A22[jc + (int64_t)i * ld] = zc{neg(uu.re), uu.im};  // -conj(u)
+          }
+        }
+      }
+    }
+    sync();
   }
+  if (P.dvim) {
+    double* dv = P.dvim + (int64_t)b * n;
+    for (int k = rank * ZNT + tid; k < n; k += ZNT * CS) dv[k] = ld2(W + k + (int64_t)k * ld).im;
+  }
+  if (CS > 1) cl.sync();  // no CTA leaves while another may still write its shared memory
 }
 
-size_t zhess_cta_smem_bytes(int nmax) { return sizeof(double) * 4 * (size_t)(nmax > 0 ? nmax : 1); }
-
-cudaError_t launch_zhess_cta(const ZHessParams& P, int grid, cudaStream_t st) {
+template <int CS>
+static cudaError_t launch_zhess_t(const ZHessParams& P, cudaStream_t st) {
   static std::atomic<uint64_t> raised{0};
-  cudaError_t e = raise_smem_limit_once((const void*)zhess_cta_kernel, raised);
+  cudaError_t e = raise_smem_limit_once((const void*)zhess_cta_kernel<CS>, raised);
   if (e != cudaSuccess) return e;
-  zhess_cta_kernel<<<grid, ZNT, zhess_cta_smem_bytes(P.nmax), st>>>(P);
-  return cudaGetLastError();
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(P.count * CS));
+  cfg.blockDim = dim3(ZNT);
+  cfg.dynamicSmemBytes = sizeof(double) * 4 * (size_t)std::max(P.n, 1);
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = CS;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, zhess_cta_kernel<CS>, P);
+}
+
+// CTAs per matrix: up to two CTAs per SM in all, and a block of 32 rows for each.
+cudaError_t launch_zhess_cta(const ZHessParams& P, cudaStream_t st) {
+  if (P.count <= 0) return cudaSuccess;
+  int dev = 0, sms = 148;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  int cs = 1;
+  while (cs < 8 && (long long)P.count * cs * 2 <= 2 * sms && P.n >= 64 * cs) cs *= 2;
+  if (cs == 1) return launch_zhess_t<1>(P, st);
+  if (cs == 2) return launch_zhess_t<2>(P, st);
+  if (cs == 4) return launch_zhess_t<4>(P, st);
+  return launch_zhess_t<8>(P, st);
 }
 
 // ---------------------------------------------------------------------------
@@ -426,21 +495,15 @@ cudaError_t zhess_large(double* Ad, int64_t lda, int n, double* taud, double* ev
   // tail: the trailing (n - c0) x (n - c0) block with the one-CTA kernel (in place, ld = lda)
   const int c0 = cend > 0 ? cend : 0;
   ZHessParams P;
-  P.W = nullptr;
-  P.W1 = reinterpret_cast<double*>(A + c0 + (int64_t)c0 * lda);
-  P.n1 = n - c0;
-  P.ld1 = lda;
+  P.W = reinterpret_cast<double*>(A + c0 + (int64_t)c0 * lda);
   P.stride = 0;
-  P.n = nullptr;
-  P.off = nullptr;
-  P.order = nullptr;
+  P.ld = lda;
+  P.n = n - c0;
   P.count = 1;
-  P.nmax = n - c0;
-  P.counter = nullptr;
   P.tau = reinterpret_cast<double*>(tau + c0);
   P.ev = ev + c0;
   P.dvim = nullptr;
-  e = launch_zhess_cta(P, 1, st);
+  e = launch_zhess_cta(P, st);
   if (e != cudaSuccess) return e;
   zdiag_im_kernel<<<(n + 255) / 256, 256, 0, st>>>(A, lda, n, dvim);
   return cudaGetLastError();

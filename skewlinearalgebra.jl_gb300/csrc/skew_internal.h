@@ -162,27 +162,18 @@ cudaError_t zeigen_tridiag(const double* ev, const double* dvim, int n, double* 
                            double* ws, cudaStream_t st);
 
 // ComplexF64 Householder tridiagonalisation (skew_complex.cu).  Complex values are
-// interleaved (re, im).  Batched: W[b] (in place, ld n[b]), tau/ev/dvim at off[b];
-// single: W == nullptr and W1/n1/ld1 (off 0).  counter == nullptr: CTA b takes
-// matrix b (grid = count), else matrices come from the counter (largest first via order).
+// interleaved (re, im).  count matrices of size n, in place: matrix b at W + b stride,
+// leading dimension ld (complex elements); tau, ev, dvim n apart.
 struct ZHessParams {
-  double* const* W;
-  double* W1;
-  int n1;
-  int64_t ld1;
-  const int32_t* n;
-  const int32_t* order;
-  const int64_t* off;
+  double* W;
+  int64_t stride, ld;
+  int n;
   int32_t count;
-  int nmax;
-  unsigned* counter;
-  int64_t stride;  // W == nullptr: matrix b at W1 + b * stride (complex elements)
   double* tau;   // complex
   double* ev;    // real subdiagonal
   double* dvim;  // imag(diag) after the reduction, or null
 };
-size_t zhess_cta_smem_bytes(int nmax);
-cudaError_t launch_zhess_cta(const ZHessParams& P, int grid, cudaStream_t st);
+cudaError_t launch_zhess_cta(const ZHessParams& P, cudaStream_t st);
 size_t zhess_large_ws_doubles(int n);
 // imag(diag(A)) of a reduced matrix into dvim
 cudaError_t launch_zdiag_im(const double* A, int64_t lda, int n, double* dvim, cudaStream_t st);

@@ -676,21 +676,15 @@ cudaError_t zhess_persistent(double* Ad, int64_t lda, int n, double* taud, doubl
   // tail: the trailing block with the one-CTA kernel, in place
   const int c0 = P.pend;
   ZHessParams T;
-  T.W = nullptr;
-  T.W1 = reinterpret_cast<double*>(A + c0 + (int64_t)c0 * lda);
-  T.n1 = n - c0;
-  T.ld1 = lda;
+  T.W = reinterpret_cast<double*>(A + c0 + (int64_t)c0 * lda);
   T.stride = 0;
-  T.n = nullptr;
-  T.off = nullptr;
-  T.order = nullptr;
+  T.ld = lda;
+  T.n = n - c0;
   T.count = 1;
-  T.nmax = n - c0;
-  T.counter = nullptr;
   T.tau = reinterpret_cast<double*>(tau + c0);
   T.ev = ev + c0;
   T.dvim = nullptr;
-  e = launch_zhess_cta(T, 1, st);
+  e = launch_zhess_cta(T, st);
   if (e != cudaSuccess) return e;
   e = launch_zdiag_im(Ad, lda, n, dvim, st);
   if (e != cudaSuccess) return e;
