@@ -50,14 +50,6 @@ __device__ __forceinline__ int2 fxp_split(double x, int e) {
   return make_int2((int)(v >> 28), (int)(v & ((1 << 28) - 1)) - (1 << 27));
 }
 
-// x 2^k exactly where it stays normal (the exponent field), else by multiplication
-__device__ __forceinline__ double fxp_ldexp(double x, int k) {
-  const int h = __double2hiint(x);
-  const int ex = ((h >> 20) & 0x7ff) + k;
-  if ((unsigned)(ex - 1) < 2045u && ((h >> 20) & 0x7ff) != 0) return __hiloint2double(h + (k << 20), __double2loint(x));
-  return scalbn(x, k);
-}
-
 // Position of entry (r, c) of a tile: quarters of 16 columns; lane 4 (r / 8) + (c % 16) / 4
 // holds 8 x 4 entries, stored pairwise so that the 32 lanes' 16-byte loads are contiguous.
 __device__ __forceinline__ int fxp_pos(int r, int c) {
@@ -691,7 +683,7 @@ __global__ void __launch_bounds__(FXP_NT, 1) fxp_panel_kernel(FxpPanel P) {
       fxp_dots(P, c, i, item, groups, R.scale, R.tau == 0.0);
     if (!fxp_barrier(P, round)) break;
     // ---- B: rows, as many threads per row as keeps every block in one round of CTAs
-    const double m2 = (R.tau == 0.0) ? 0.0 : fxp_ldexp(R.scale, -k);
+    const double m2 = (R.tau == 0.0) ? 0.0 : oz_ldexp(R.scale, -k);
     int nfb;
     if ((m + 15) / 16 <= (int)gridDim.x) {
       nfb = (m + 15) / 16;
@@ -786,14 +778,14 @@ struct FxpUpdate {
     for (int u = 0; u < NV; u++) {
       double x = 0.0;
       if (l0 + u < nbp) x = vside ? A[q + r + (int64_t)(p + l0 + u) * lda] : w.W[(size_t)(l0 + u) * n + q + r];
-      if (vside) x = fxp_ldexp(x, k);
+      if (vside) x = oz_ldexp(x, k);
       v[u] = (vside && !left) ? neg(x) : x;
     }
   }
   __device__ void loadA(int i, int s, int kk, double (&v)[8]) const { load<8>(i, s * OZ_K + kk, true, v); }
   __device__ void loadB(int j, int s, int kk, double (&v)[4]) const { load<4>(j, s * OZ_K + kk, false, v); }
   __device__ void store(int i, int j, double x) const {
-    if (i > j) A[q + i + (int64_t)(q + j) * lda] += fxp_ldexp(x, -k);
+    if (i > j) A[q + i + (int64_t)(q + j) * lda] += oz_ldexp(x, -k);
   }
   __device__ void timeout() const { w.sync[1] = 1u; }
 };
