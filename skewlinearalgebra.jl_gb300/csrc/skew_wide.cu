@@ -14,8 +14,8 @@
 // grid barriers per column), fxp_exps_kernel, fxp_update_kernel.  The last columns go to the
 // one-CTA kernel of skew_batch.cu.  Sums of the tiles are formed in a fixed order.
 //
-// Whole reduction: n = 1025 19.0 -> 17.4 ms, 2048 51.0 -> 37.6, 4096 195 -> 96, 8192 929 -> 366
-// (panels 305, update 52, packing 5).
+// Whole reduction: n = 2048 51.0 -> 35.4 ms, 8192 929 -> 335 (panels 284, update 43,
+// packing 5).
 //
 // Eigenvalues in the QR's deflation order (n <= 1024) keep the kernels of skew_blocked.cu
 // and skew_cluster.cu: the order depends on the last bits of the tridiagonal.
@@ -40,6 +40,7 @@ constexpr int FXP_SLOTS = 3;                  // quarter tiles in flight per war
 constexpr int FXP_QUARTER = FXP_TILE / 4 * 8; // bytes
 constexpr int FXP_DOT_ROWS = 256;             // rows and columns of a panel dot item: 8 x 4 FMAs per lane
 constexpr int FXP_DOT_COLS = 4;
+constexpr int FXP_CTAS = 1024;                // largest grid of the panel kernel
 // shared memory: quarter tiles, x of a tile's rows and columns per warp, barriers
 constexpr int FXP_SMEM = FXP_NW * (FXP_SLOTS * FXP_QUARTER + 2 * FXP_T * 8 + FXP_SLOTS * 8);
 constexpr long long FXP_POLLS = 1LL << 24;    // default polls of a grid barrier: seconds
@@ -64,7 +65,7 @@ struct FxpWs {
   double* rowpart;  // tile columns x n: shares of A22 v from tiles right of (and on) the diagonal
   double* colpart;  // slots x n: shares of the mirrored tiles
   double* upart;    // row chunks x 2 FXP_NB
-  double* sspart;
+  double* sspart;   // one per CTA
   int *ev, *ew;     // largest exponents of the panel's rows of V and W
   unsigned* sync;   // [0] barrier arrivals, [1] error, [2] W's largest exponent
 };
@@ -87,7 +88,7 @@ static size_t fxp_carve(FxpWs* w, double* base, int n) {
   x.rowpart = take(T * n);
   x.colpart = take((T + 2) * n);
   x.upart = take(((size_t)n / FXP_DOT_ROWS + 1) * 2 * FXP_NB);
-  x.sspart = take((size_t)n / 16 + 1);
+  x.sspart = take(FXP_CTAS);
   x.ev = (int*)take((size_t)n / 2 + 1);
   x.ew = (int*)take((size_t)n / 2 + 1);
   x.sync = (unsigned*)take(4);
@@ -103,7 +104,7 @@ size_t wide_ws_doubles(int n) { return n > kWideMin ? fxp_carve(nullptr, nullptr
 __host__ __device__ __forceinline__ int fxp_first(int T, int tj) { return tj * T - tj * (tj - 1) / 2; }
 
 __device__ __forceinline__ void fxp_tile_at(int T, int t, int* ti, int* tj) {
-  int j = (int)(T + 0.5 - sqrt((T + 0.5) * (T + 0.5) - 2.0 * t));
+  int j = (int)(T + 0.5f - sqrtf((T + 0.5f) * (T + 0.5f) - 2.0f * t));  // corrected below
   j = max(0, min(T - 1, j));
   while (j > 0 && fxp_first(T, j) > t) j--;
   while (j + 1 < T && fxp_first(T, j + 1) <= t) j++;
@@ -158,8 +159,10 @@ struct FxpPanel {
   int skip_cta;
 };
 
-// Grid barrier on a monotonic arrival counter; false if it gave up or another CTA did.
-__device__ bool fxp_barrier(const FxpPanel& P, unsigned& round) {
+// Grid barrier on a monotonic arrival counter; false if it gave up or an error was set
+// before it.  pre() is run by thread 0 between the CTA's own barrier and its arrival.
+template <class Pre>
+__device__ bool fxp_barrier(const FxpPanel& P, unsigned& round, Pre pre) {
   __shared__ int s_ok;
   __syncthreads();
   round++;
@@ -173,7 +176,9 @@ __device__ bool fxp_barrier(const FxpPanel& P, unsigned& round) {
       while (!*err && ++it <= P.poll_limit) __nanosleep(100);
       ok = 0;
     } else {
+      pre();
       asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(cnt) : "memory");
+      const unsigned before = *err;  // looked at after the wait, which hides the read
       long long it = 0;
       for (;;) {
         unsigned v;
@@ -189,8 +194,9 @@ __device__ bool fxp_barrier(const FxpPanel& P, unsigned& round) {
           break;
         }
       }
+      ok = ok && !before;
     }
-    s_ok = ok && !*err;
+    s_ok = ok;
   }
   __syncthreads();
   return s_ok != 0;
@@ -463,20 +469,30 @@ __device__ __forceinline__ void fxp_dots(const FxpPanel& P, int c, int i, int it
   if (!(lane & 7) && d < 2 * i) P.w.upart[(size_t)chunk * 2 * FXP_NB + (d < i ? d : FXP_NB + d - i)] = s[0];
 }
 
-// y of one row 2^k (partial sums of the tiles), TPR threads per row: thread g's share
+// y of one row 2^k (partial sums of the tiles), TPR threads per row: thread g's share, eight
+// reads at a time
 template <int TPR>
 __device__ __forceinline__ double fxp_row_sum(const FxpPanel& P, int row, int g) {
   const int n = P.n, tr = (row - P.p - 1) / FXP_T;
-  double y0 = 0.0, y1 = 0.0;
-  int q = g;
-  for (; q + TPR <= tr; q += 2 * TPR) {
-    y0 += __ldcg(P.w.rowpart + (size_t)q * n + row);
-    y1 += __ldcg(P.w.rowpart + (size_t)(q + TPR) * n + row);
-  }
-  if (q <= tr) y0 += __ldcg(P.w.rowpart + (size_t)q * n + row);
   const int f = fxp_first(P.T, tr), slots = (f + P.T - tr - 1) / P.per - f / P.per + 1;
-  for (q = g; q < slots; q += TPR) y1 -= __ldcg(P.w.colpart + (size_t)q * n + row);
-  return y0 + y1;
+  double y[2] = {0.0, 0.0};
+  for (int q = g; q <= tr; q += 8 * TPR) {
+    double t[8];
+#pragma unroll
+    for (int z = 0; z < 8; z++) t[z] = (q + z * TPR <= tr) ? __ldcg(P.w.rowpart + (size_t)(q + z * TPR) * n + row) : 0.0;
+#pragma unroll
+    for (int z = 0; z < 8; z++)
+      if (q + z * TPR <= tr) y[z & 1] += t[z];
+  }
+  for (int q = g; q < slots; q += 4 * TPR) {
+    double t[4];
+#pragma unroll
+    for (int z = 0; z < 4; z++) t[z] = (q + z * TPR < slots) ? __ldcg(P.w.colpart + (size_t)(q + z * TPR) * n + row) : 0.0;
+#pragma unroll
+    for (int z = 0; z < 4; z++)
+      if (q + z * TPR < slots) y[1] -= t[z];
+  }
+  return y[0] + y[1];
 }
 
 // What the rows of a step share: sums of the panel dots (u1, u2) and row c + 1 of W and A.
@@ -486,48 +502,64 @@ struct FxpShared {
   double red[FXP_NW];
 };
 
+// What a thread reads for it: two threads per dot, even and odd chunks; the last warp, which
+// has the fewest rows, also row c + 1.
+struct FxpHead {
+  double up[8], w[2], a[2];
+};
+__device__ __forceinline__ void fxp_head_load(const FxpPanel& P, int c, int i, int chunks, FxpHead& L) {
+  const int tid = threadIdx.x, lane = tid & 31, n = P.n, r0 = c + 1;
+  const int d = tid >> 1, h = tid & 1;
+  const bool in = (d & (FXP_NB - 1)) < i;
+#pragma unroll
+  for (int z = 0; z < 8; z++)
+    L.up[z] = (in && h + 2 * z < chunks) ? __ldcg(P.w.upart + (size_t)(h + 2 * z) * 2 * FXP_NB + d) : 0.0;
+#pragma unroll
+  for (int t = 0; t < 2; t++) {
+    const int j = lane + 32 * t;
+    L.w[t] = L.a[t] = 0.0;
+    if (tid >= FXP_NT - 32 && j < i) {
+      L.w[t] = __ldcg(P.w.W + (size_t)j * n + r0);
+      L.a[t] = __ldcg(P.A + r0 + (int64_t)(P.p + j) * P.lda);
+    }
+  }
+}
+
 // Fills it, by the whole CTA.  m2 = scale 2^-k.
 __device__ __forceinline__ void fxp_step_shared(const FxpPanel& P, int c, int i, int chunks, const FxpRefl& R,
-                                                double m2, FxpShared& H) {
-  const int tid = threadIdx.x, lane = tid & 31, n = P.n, p = P.p, r0 = c + 1;
-  // warp 0's loads of row c + 1 go out before the sums of the dots
-  double acc = 0.0, wv[2] = {0.0, 0.0}, av[2] = {0.0, 0.0};
-  if (tid < 32) {
-#pragma unroll
-    for (int t = 0; t < 2; t++) {
-      const int j = lane + 32 * t;
-      if (j < i) {
-        wv[t] = __ldcg(P.w.W + (size_t)j * n + r0);
-        av[t] = __ldcg(P.A + r0 + (int64_t)(p + j) * P.lda);
-      }
-    }
-    acc = fxp_row_sum<32>(P, r0, lane);
-  }
-  // two threads per dot, even and odd chunks
-  const int d = tid & (2 * FXP_NB - 1), h = tid / (2 * FXP_NB);
+                                                double m2, const FxpHead& L, FxpShared& H) {
+  const int tid = threadIdx.x, lane = tid & 31, r0 = c + 1;
+  const int d = tid >> 1, h = tid & 1;
   double s0 = 0.0, s1 = 0.0;
   if ((d & (FXP_NB - 1)) < i) {
-    int q = h;
-    for (; q + 2 < chunks; q += 4) {
-      s0 += __ldcg(P.w.upart + (size_t)q * 2 * FXP_NB + d);
-      s1 += __ldcg(P.w.upart + (size_t)(q + 2) * 2 * FXP_NB + d);
+#pragma unroll
+    for (int z = 0; z < 8; z++)
+      if (h + 2 * z < chunks) (z & 1 ? s1 : s0) += L.up[z];
+    for (int q = h + 16; q < chunks; q += 16) {
+      double t[8];
+#pragma unroll
+      for (int z = 0; z < 8; z++)
+        t[z] = (q + 2 * z < chunks) ? __ldcg(P.w.upart + (size_t)(q + 2 * z) * 2 * FXP_NB + d) : 0.0;
+#pragma unroll
+      for (int z = 0; z < 8; z++)
+        if (q + 2 * z < chunks) (z & 1 ? s1 : s0) += t[z];
     }
-    if (q < chunks) s0 += __ldcg(P.w.upart + (size_t)q * 2 * FXP_NB + d);
     s0 += s1;
   }
-  if (h) H.su[d] = s0;
+  s0 += __shfl_xor_sync(0xffffffffu, s0, 1);
+  if (!h) H.su[d] = s0;
+  const bool head = tid >= FXP_NT - 32;
+  double acc = head ? fxp_row_sum<32>(P, r0, lane) : 0.0;
   __syncthreads();
-  if (!h) H.su[d] += s0;
-  __syncthreads();
-  if (tid < 32) {  // row c + 1 of W, which every row's column update needs
+  if (head) {  // row c + 1 of W, which every row's column update needs
     acc *= m2;
 #pragma unroll
     for (int t = 0; t < 2; t++) {
       const int j = lane + 32 * t;
       if (j < i) {
-        acc = fma(av[t], H.su[j], fma(-wv[t], H.su[FXP_NB + j], acc));
-        H.Wrow[j] = wv[t];
-        H.Arow[j] = av[t];
+        acc = fma(L.a[t], H.su[j], fma(-L.w[t], H.su[FXP_NB + j], acc));
+        H.Wrow[j] = L.w[t];
+        H.Arow[j] = L.a[t];
       }
     }
     acc = warp_sum(acc);
@@ -540,20 +572,22 @@ __device__ __forceinline__ void fxp_step_shared(const FxpPanel& P, int c, int i,
 }
 
 // Rows of the panel step: W[:, i], v into column c, the deferred update of column c + 1 and
-// the norm partials of its rows below the subdiagonal.  A block's loads go out before the
-// shared sums are formed.
+// the sum of squares of its rows below the subdiagonal (ssp: this thread's share).  Row blocks
+// go to the warps CTA-minor, so that TPR chosen for one block per quarter SM spreads the FP64
+// work evenly.  A block's loads go out before the shared sums are formed.
 template <int TPR>
 __device__ void fxp_rows(const FxpPanel& P, int c, int i, int chunks, bool last, const FxpRefl& R, double m2,
-                         FxpShared& H) {
-  constexpr int ROWS = FXP_NT / TPR, NJ = FXP_NB / TPR;
+                         FxpShared& H, double& ssp) {
+  constexpr int RPW = 32 / TPR, NJ = FXP_NB / TPR;
   double* A = P.A;
   const int64_t lda = P.lda;
-  const int tid = threadIdx.x, n = P.n, p = P.p;
-  const int nfb = (n - c - 1 + ROWS - 1) / ROWS;
-  for (int fb = blockIdx.x; fb < nfb; fb += gridDim.x) {
-    const int row = c + 1 + fb * ROWS + tid / TPR, g = tid % TPR;
-    const bool valid = row < n;
-    double aj[NJ], wj[NJ];
+  const int lane = threadIdx.x & 31, n = P.n, p = P.p, g = lane % TPR;
+  const int nrb = (n - c - 1 + RPW - 1) / RPW;
+  const int rb0 = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+  double aj[NJ], wj[NJ], vr, y, next;  // next: column c + 1 as it was at the panel's start
+  auto load = [&](int rb) {
+    const int row = c + 1 + rb * RPW + lane / TPR;
+    const bool valid = rb < nrb && row < n;
 #pragma unroll
     for (int t = 0; t < NJ; t++) {
       const int j = g + TPR * t;
@@ -564,25 +598,32 @@ __device__ void fxp_rows(const FxpPanel& P, int c, int i, int chunks, bool last,
         wj[t] = __ldcg(P.w.W + (size_t)j * n + row);
       }
     }
-    double vr = 0.0, acc = 0.0, next = 0.0;  // next: column c + 1 as it was at the panel's start
+    vr = y = next = 0.0;
     if (valid) {
       next = (row >= c + 2) ? __ldcg(A + row + (int64_t)(c + 1) * lda) : 0.0;
       vr = (R.tau == 0.0 || row == c + 1) ? 0.0 : __ldcg(A + row + (int64_t)c * lda);
-      acc = fxp_row_sum<TPR>(P, row, g);
+      y = fxp_row_sum<TPR>(P, row, g);
     }
-    if (fb == blockIdx.x) fxp_step_shared(P, c, i, chunks, R, m2, H);
-    acc *= m2;
-    if (g == 0) acc += next;  // v[c + 1] = 1
-    double acc1 = 0.0;
+  };
+  FxpHead L;
+  fxp_head_load(P, c, i, chunks, L);
+  load(rb0);
+  fxp_step_shared(P, c, i, chunks, R, m2, L, H);
+  ssp = 0.0;
+  for (int rb = rb0; rb < nrb; rb += gridDim.x * FXP_NW) {
+    if (rb != rb0) load(rb);
+    const int row = c + 1 + rb * RPW + lane / TPR;
+    const bool valid = row < n;
+    double acc = y * m2, acc1 = (g == 0) ? next : 0.0;  // v[c + 1] = 1
 #pragma unroll
     for (int t = 0; t < NJ; t++) {
       const int j = g + TPR * t;
       if (j < i) {
         acc = fma(aj[t], H.su[j], acc);
-        acc1 = fma(wj[t], H.su[FXP_NB + j], acc1);
+        acc1 = fma(-wj[t], H.su[FXP_NB + j], acc1);
       }
     }
-    acc -= acc1;
+    acc += acc1;
 #pragma unroll
     for (int o = 1; o < TPR; o <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
     double wri = (R.tau == 0.0) ? 0.0 : R.tau * acc;
@@ -592,45 +633,34 @@ __device__ void fxp_rows(const FxpPanel& P, int c, int i, int chunks, bool last,
       P.w.W[(size_t)i * n + row] = wri;
       A[row + (int64_t)c * lda] = vr;
     }
-    double ssp = 0.0;
-    if (!last) {
-      double uu = 0.0, uu1 = 0.0;
+    if (last) continue;
+    double uu = 0.0, uu1 = 0.0;
 #pragma unroll
-      for (int t = 0; t < NJ; t++) {
-        const int j = g + TPR * t;
-        if (j < i) {
-          uu = fma(aj[t], H.Wrow[j], uu);
-          uu1 = fma(wj[t], H.Arow[j], uu1);
-        }
+    for (int t = 0; t < NJ; t++) {
+      const int j = g + TPR * t;
+      if (j < i) {
+        uu = fma(aj[t], H.Wrow[j], uu);
+        uu1 = fma(-wj[t], H.Arow[j], uu1);
       }
-      uu -= uu1;
-      if (i % TPR == g) uu = fma(vr, H.Wrow[i], fma(-wri, H.Arow[i], uu));
+    }
+    if (i % TPR == g) uu = fma(vr, H.Wrow[i], fma(-wri, H.Arow[i], uu));
+    uu += uu1;
 #pragma unroll
-      for (int o = 1; o < TPR; o <<= 1) uu += __shfl_xor_sync(0xffffffffu, uu, o);
-      if (valid && row >= c + 2 && g == 0) {
-        const double anew = next + uu;
-        A[row + (int64_t)(c + 1) * lda] = anew;
-        if (row >= c + 3) ssp = anew * anew;
-      }
-      // the block's sum of squares: lanes g = 0 of each warp, then the warps
-#pragma unroll
-      for (int o = 16; o >= TPR; o >>= 1) ssp += __shfl_xor_sync(0xffffffffu, ssp, o);
-      if ((tid & 31) == 0) H.red[tid >> 5] = ssp;
-      __syncthreads();
-      if (tid < 32) {
-        double s = (tid < FXP_NW) ? H.red[tid] : 0.0;
-#pragma unroll
-        for (int o = FXP_NW / 2; o >= 1; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (tid == 0) P.w.sspart[fb] = s;
-      }
-      __syncthreads();
+    for (int o = 1; o < TPR; o <<= 1) uu += __shfl_xor_sync(0xffffffffu, uu, o);
+    if (valid && row >= c + 2 && g == 0) {
+      const double anew = next + uu;
+      A[row + (int64_t)(c + 1) * lda] = anew;
+      if (row >= c + 3) ssp = fma(anew, anew, ssp);
     }
   }
 }
 
-// n = 8192, first panel, per column: the product 41 us (268 MB, 6.5 TB/s; 115 us on the
-// FP64 pipe from the full square), rows 15, the two barriers' waits 10, the next reflector 2; at
-// m = 4096, where the tiles stay in L2, 12, 9, 6 and 2.
+// n = 8192, first panel, per column: the product 44 us (268 MB, 6.1 TB/s; 115 us on the
+// FP64 pipe from the full square), rows 15, the two barriers' waits 12, the next reflector 3; at
+// m = 3072, where the tiles stay in L2, 7, 8, 8 and 3.  Loads in batches before the sums that
+// wait for them and row blocks dealt to the warps of all CTAs took rows and the wait behind
+// them from 24 to 18 us (from 14 to 11 at m = 3072).  At small m the product is the latency of
+// one tile (7 us): its 768 IMADs per warp take 3, the rest is reading x, shuffles, conversions.
 __global__ void __launch_bounds__(FXP_NT, 1) fxp_panel_kernel(FxpPanel P) {
   extern __shared__ __align__(128) unsigned char fsm[];
   __shared__ double red[FXP_NW];
@@ -681,28 +711,34 @@ __global__ void __launch_bounds__(FXP_NT, 1) fxp_panel_kernel(FxpPanel P) {
     const int chunks = (m + FXP_DOT_ROWS - 1) / FXP_DOT_ROWS;
     for (int item = nwarps - 1 - gw; item < groups * chunks; item += nwarps)
       fxp_dots(P, c, i, item, groups, R.scale, R.tau == 0.0);
-    if (!fxp_barrier(P, round)) break;
-    // ---- B: rows, as many threads per row as keeps every block in one round of CTAs
+    if (!fxp_barrier(P, round, []() {})) break;
+    // ---- B: rows, as many threads per row as leaves one row block per quarter SM
     const double m2 = (R.tau == 0.0) ? 0.0 : oz_ldexp(R.scale, -k);
-    int nfb;
-    if ((m + 15) / 16 <= (int)gridDim.x) {
-      nfb = (m + 15) / 16;
-      fxp_rows<16>(P, c, i, chunks, last, R, m2, H);
-    } else if ((m + 31) / 32 <= (int)gridDim.x) {
-      nfb = (m + 31) / 32;
-      fxp_rows<8>(P, c, i, chunks, last, R, m2, H);
-    } else {
-      nfb = (m + 63) / 64;
-      fxp_rows<4>(P, c, i, chunks, last, R, m2, H);
-    }
+    const int quarters = 4 * gridDim.x;
+    double ssp;
+    if (m <= quarters)
+      fxp_rows<32>(P, c, i, chunks, last, R, m2, H, ssp);
+    else if (m <= 2 * quarters)
+      fxp_rows<16>(P, c, i, chunks, last, R, m2, H, ssp);
+    else if (m <= 4 * quarters)
+      fxp_rows<8>(P, c, i, chunks, last, R, m2, H, ssp);
+    else
+      fxp_rows<4>(P, c, i, chunks, last, R, m2, H, ssp);
     if (last) break;
-    if (!fxp_barrier(P, round)) break;
+    ssp = warp_sum(ssp);
+    if (lane == 0) H.red[w] = ssp;
+    static_assert(FXP_NW == 8, "a tree of eight sums");
+    if (!fxp_barrier(P, round, [&]() {
+          const double* x = H.red;
+          P.w.sspart[blockIdx.x] = ((x[0] + x[1]) + (x[2] + x[3])) + ((x[4] + x[5]) + (x[6] + x[7]));
+        }))
+      break;
     // reflector c + 1, identically in every CTA, formed by one lane
     const int c1 = c + 1;
     if (w == 0) {
       const double alpha = __ldcg(A + (c1 + 1) + (int64_t)c1 * lda);
       double ss = 0.0;
-      for (int t = lane; t < nfb; t += 32) ss += __ldcg(P.w.sspart + t);
+      for (int t = lane; t < (int)gridDim.x; t += 32) ss += __ldcg(P.w.sspart + t);
       ss = warp_sum(ss);
       if (lane == 0) {
         s_scal = ss_needs_scaling(ss) ? 1 : 0;
@@ -825,8 +861,8 @@ cudaError_t wide_hessenberg(double* A, int64_t lda, int n, double* tau, double* 
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fxp_panel_kernel, FXP_NT, FXP_SMEM);
   if (e != cudaSuccess) return e;
   if (occ < 1) return cudaErrorNotSupported;
-  int grid = sms, tail = FXP_TAIL;
-  if (T.persist_ctas > 0) grid = std::max(1, std::min(sms, T.persist_ctas));
+  int grid = std::min(sms, FXP_CTAS), tail = FXP_TAIL;
+  if (T.persist_ctas > 0) grid = std::max(1, std::min(grid, T.persist_ctas));
   if (T.persist_tail > 0) tail = std::max(32, std::min(FXP_TAIL, T.persist_tail));
   const int nb = std::max(8, std::min(FXP_NB, T.persist_nb));
   const int pend = n - tail;
