@@ -174,7 +174,8 @@ __device__ double group_multisect(double lo, double hi, int target, double absto
 // instruction per 64 cycles of a sub-partition, whatever its active lanes): two
 // instructions per row from the squares e2 = e^2 (three with a diagonal), where the
 // pivot form q_i = d_i - x - e^2 / q_{i-1} takes a division and about twelve.  The
-// multisection of 512 problems of n = 32 .. 512: 86.4 -> 23.4 ms; n = 2048: 16.9 -> 4.3 ms.
+// multisection of 512 problems of n = 32 .. 512: 86.4 -> 23.4 ms; n = 2048: 16.9 -> 4.3 ms
+// (3.4 with group_rootsect's fewer steps).
 // Each step's rounding is a relative change of its (d_i - x) and e^2, so with a zero
 // diagonal tiny eigenvalues keep their relative accuracy, as with the pivots.  A zero
 // p_i stands for a pivot a hair below zero and is counted, as the pivot form's -pivmin
@@ -182,8 +183,13 @@ __device__ double group_multisect(double lo, double hi, int target, double absto
 // the middle of the exponent range whenever both lie outside 2^-256 .. 2^256; d, e2 and
 // x come scaled to a spectrum within [-1, 1], so one step cannot leave the range.
 // d(i), e2(i): entry i of the scaled diagonal (dx(i) = d_i - x) and of the squares.
+struct SturmVal {
+  int c;     // eigenvalues below x
+  double m;  // p_n(x) = m 2^k
+  int k;
+};
 template <class DX, class E2>
-__device__ __forceinline__ int sturm_products(int n, DX dx, E2 e2) {
+__device__ __forceinline__ SturmVal sturm_products(int n, DX dx, E2 e2) {
   // p == 0: the other sign than the entry before it (high word hb), 2^-400 of its size
   auto settle = [](double& p, int& h, int hb) {
     if (((h << 1) | __double2loint(p)) == 0) {
@@ -194,7 +200,7 @@ __device__ __forceinline__ int sturm_products(int n, DX dx, E2 e2) {
   double p0 = 1.0, p1 = dx(0);
   int h1 = __double2hiint(p1);
   settle(p1, h1, 0x3ff00000);
-  int c = (unsigned)h1 >> 31;
+  int c = (unsigned)h1 >> 31, k = 0;
   for (int i = 1; i < n; i++) {
     double p2 = fma(dx(i), p1, neg(e2(i - 1) * p0));
     int h2 = __double2hiint(p2);
@@ -203,6 +209,7 @@ __device__ __forceinline__ int sturm_products(int n, DX dx, E2 e2) {
     const int top = max(h2 & 0x7fffffff, h1 & 0x7fffffff);
     if ((unsigned)(top - 0x2ff00000) > 0x20000000u) {  // the pair lies outside 2^-256 .. 2^256
       const double f = (top < 0x3ff00000) ? 0x1p+500 : 0x1p-500;
+      k += (top < 0x3ff00000) ? -500 : 500;
       p1 *= f;
       p2 *= f;
       const int s2 = h2 & 0x80000000;
@@ -216,7 +223,106 @@ __device__ __forceinline__ int sturm_products(int n, DX dx, E2 e2) {
     p1 = p2;
     h1 = h2;
   }
-  return c;
+  return SturmVal{c, p1, k};
+}
+
+// |a / b| of two values m 2^k
+__device__ __forceinline__ double sturm_ratio(double am, int ak, double bm, int bk) {
+  const int d = max(-1000, min(1000, ak - bk));
+  return fabs(am / bm) * __hiloint2double((1023 + d) << 20, 0);
+}
+
+// group_multisect where the count comes with the value of the characteristic polynomial:
+// once one eigenvalue is left between two counted points, the secant through the
+// polynomial's values there says where it lies.  The points are then
+//   p = 1: the secant's root, and after it twice as far from the new end as the next secant's
+//          root, so that the other end follows;
+//   p > 1: pairs around the secant's root at distances of 2^-s of the interval (p = 2, 4: s
+//          doubles while it succeeds).
+// The counts alone decide which points become the new interval, so it keeps the bracket
+// count(lo) <= target < count(hi) of group_multisect and ends at the same width.  Guesses that
+// brought less than even division (another eigenvalue close outside) are followed by even
+// steps, more after each failure; so is the end, within four final widths.
+// Bound by the FP64 pipe and its latency: two FMAs per row and step, so the steps count: 19 to
+// 24 instead of 53 with one lane per eigenvalue, 11 to 13 instead of 23 with 4, 8 to 10 instead
+// of 13 with 16, 8 instead of 11 with 32.
+template <class Eval>
+__device__ double group_rootsect(double lo, double hi, int target, double abstol, int p, bool active, Eval eval) {
+  const int lane = threadIdx.x & 31;
+  const int g = lane / p, gl = lane - g * p;
+  const unsigned gmask = (p == 32) ? 0xffffffffu : (((1u << p) - 1u) << (g * p));
+  const double inv = 1.0 / (double)(p + 1);
+  const double enough = (p == 1) ? 0.25 : inv;  // of the interval a guess (p = 1: two) may leave
+  const int gap = (p == 8) ? 5 : (p == 16 ? 4 : 3);
+  const int pair = (gl < p / 2) ? gl : p - 1 - gl;
+  SturmVal vl{-1, 0.0, 0}, vh{-1, 0.0, 0};  // at lo and hi, once counted there
+  int wait = 0, fails = 0, s = 3;
+  int moved = 0;  // p = 1: the end that the first guess of two moved (1: hi, 2: lo)
+  double wref = 0.0;
+  bool run = active;
+  for (int it = 0; it < 256; it++) {
+    const double w = hi - lo;
+    const double tol = fmax(2.220446049250313e-16 * fmax(fabs(lo), fabs(hi)), abstol);
+    if (run && !(w > tol)) run = false;
+    if (!__any_sync(0xffffffffu, run)) break;
+    bool guess = vl.c >= 0 && vh.c == vl.c + 1 && w > 4.0 * tol;
+    if (!guess) moved = 0;
+    if (guess && moved == 0) {
+      if (wait > 0) {
+        wait--;
+        guess = false;
+      } else if (wref > 0.0 && w > wref * enough) {
+        wait = min(2 * fails, 8);
+        fails++;
+        s = 3;
+        wref = 0.0;
+        guess = false;
+      } else {
+        if (wref > 0.0) {
+          fails = 0;
+          s = min(2 * s, 24);
+        }
+        wref = w;
+      }
+    }
+    double x = lo + w * ((double)(gl + 1) * inv);
+    if (run && guess) {
+      double root = lo + w / (1.0 + sturm_ratio(vh.m, vh.k, vl.m, vl.k));
+      if (p == 1) {
+        if (moved == 2) root += fmax(root - lo, 0.25 * tol);
+        if (moved == 1) root -= fmax(hi - root, 0.25 * tol);
+        x = fmin(fmax(root, lo + 0.5 * tol), hi - 0.5 * tol);
+      } else {
+        const int e = (p <= 4) ? s * (pair + 1) : 2 + gap * pair;  // at most 48
+        const double o = fmax(w * __hiloint2double((1023 - e) << 20, 0), 0.45 * tol);
+        x = (gl < p / 2) ? fmax(lo, root - o) : fmin(hi, root + o);
+      }
+    }
+    SturmVal v{0, 0.0, 0};
+    if (run) v = eval(x);
+    const bool below = run ? (v.c <= target) : true;
+    const unsigned bits = __ballot_sync(0xffffffffu, below) & gmask;
+    const unsigned above = ~bits & gmask;  // points whose count exceeds the target
+    const int j = above ? (__ffs(above) - 1 - g * p) : p;  // first such point (p: none)
+    const int sl = g * p + max(j - 1, 0), sh = g * p + min(j, p - 1);
+    const double xl = __shfl_sync(0xffffffffu, x, sl), xh = __shfl_sync(0xffffffffu, x, sh);
+    const SturmVal nl{__shfl_sync(0xffffffffu, v.c, sl), __shfl_sync(0xffffffffu, v.m, sl),
+                      __shfl_sync(0xffffffffu, v.k, sl)};
+    const SturmVal nh{__shfl_sync(0xffffffffu, v.c, sh), __shfl_sync(0xffffffffu, v.m, sh),
+                      __shfl_sync(0xffffffffu, v.k, sh)};
+    if (run) {
+      if (p == 1) moved = (guess && moved == 0) ? j + 1 : 0;
+      if (j > 0) {
+        lo = xl;
+        vl = nl;
+      }
+      if (j < p) {
+        hi = xh;
+        vh = nh;
+      }
+    }
+  }
+  return 0.5 * (lo + hi);
 }
 
 // The power of two that brings a spectrum within [-bound, bound] into [-1, 1].

@@ -670,7 +670,7 @@ __global__ void zbisect_kernel(const double* __restrict__ dg, const double* __re
       return v * v;
     });
   };
-  const double x = group_multisect(lo, hi, k, 2.220446049250313e-16 * fmax(fabs(lo), fabs(hi)), p, active, count);
+  const double x = group_rootsect(lo, hi, k, 2.220446049250313e-16 * fmax(fabs(lo), fabs(hi)), p, active, count);
   if (active && gl == 0) {
     if (mu) mu[mb * n + k] = x;
     vals_im[mb * n + k] = neg(x);

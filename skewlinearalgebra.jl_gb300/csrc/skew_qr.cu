@@ -230,7 +230,7 @@ __device__ __forceinline__ void stage_squares(const double* __restrict__ e, int 
   }
   __syncthreads();
 }
-__device__ __forceinline__ int sturm_zero_diag(const double* __restrict__ e, int n, double scale, const double* sq,
+__device__ __forceinline__ SturmVal sturm_zero_diag(const double* __restrict__ e, int n, double scale, const double* sq,
                                                double x) {
   const double nx = neg(x * scale);
   if (n <= STURM_STAGE) return sturm_products(n, [&](int) { return nx; }, [&](int i) { return sq[i]; });
@@ -255,7 +255,7 @@ __global__ void bisect_kernel_dev(const double* __restrict__ e, int n, const dou
   const double bound = bp[0], pivmin = bp[1], scale = sturm_scale(bound);
   stage_squares(e, n, scale, sq);
   const bool active = gid < h;
-  const double x = group_multisect(0.0, bound, n - 1 - (active ? gid : 0), 4.0 * pivmin, p, active,
+  const double x = group_rootsect(0.0, bound, n - 1 - (active ? gid : 0), 4.0 * pivmin, p, active,
                                    [&](double y) { return sturm_zero_diag(e, n, scale, sq, y); });
   if (active && gl == 0) {
     vals[gid] = x;
@@ -329,7 +329,7 @@ __global__ void bisect_batch_kernel(const double* __restrict__ e_g, int n, const
   const double bound = bp[0], pivmin = bp[1], scale = sturm_scale(bound);
   stage_squares(e, n, scale, sq);
   const bool active = gid < h;
-  const double x = group_multisect(0.0, bound, n - 1 - (active ? gid : 0), 4.0 * pivmin, p, active,
+  const double x = group_rootsect(0.0, bound, n - 1 - (active ? gid : 0), 4.0 * pivmin, p, active,
                                    [&](double y) { return sturm_zero_diag(e, n, scale, sq, y); });
   if (active && gl == 0) {
     vals[gid] = x;
