@@ -41,6 +41,7 @@ struct Bucket {
   int begin, end, nmax, smem_matrix, grid, nt;
   int64_t gws_slot;  // doubles per CTA slot (global bucket)
   int split = 0;     // > begin: the work median of the slice (two regions, see batch_kernel)
+  int grid_wide = 0;  // > 0: CTAs of 16 warps, one per SM (functions of the matrices)
   size_t gws_off;    // offset of the bucket's slots in the plan workspace (doubles)
 };
 
@@ -617,6 +618,20 @@ int skew_batch_plan_create(skew_handle_t h, const int64_t* n, int64_t count, ske
       B.split = (int)std::max<int64_t>(q, t + 1);
     }
     B.grid = (int)std::min<int64_t>((int64_t)h->sms * occ, u - t);
+    // One CTA of 16 warps per SM instead of two of 8 where the largest matrix, not the sum,
+    // sets the time: it alone keeps an SM longer (n = 512: 31 ms against 43), and finishes
+    // a batch of sizes 100 .. 512 in 0.61 of the time (304 matrices, 33 ms against 55).
+    // Measured over counts 16 .. 450: from sizes 384 on never slower (0.65 .. 1.01); below,
+    // faster (0.65 .. 0.97) while slots nmax^3 >= 1.7 sum n^3 and up to 1.5 times slower
+    // under that (200 of n = 100).  The row sums are split differently, so only the functions'
+    // eigenpairs take it: eigenvalues follow the QR's deflation order, and log|Pf| is the
+    // same to the last bit whatever else is in its batch.
+    if (!B.smem_matrix && B.nt == 256) {
+      double total = 0.0;
+      for (int64_t q = t; q < u; q++) total += std::pow((double)P->n_host[order[q]], 3.0);
+      if (B.nmax >= 384 || 2.0 * h->sms * std::pow((double)B.nmax, 3.0) >= 1.7 * total)
+        B.grid_wide = std::min(B.grid, h->sms * batch_occupancy(B.nmax, false, 512));
+    }
     B.gws_slot = B.smem_matrix ? 0 : (int64_t)B.nmax * (B.nmax | 1);
     B.gws_off = gws_total;
     gws_total += (size_t)B.gws_slot * B.grid;
@@ -723,7 +738,7 @@ static int pfgrad_ws(skew_batch_plan_t P) {
 static int run_buckets(skew_batch_plan_t P, const double* const* A, double* logpf, double* sign,
                        double* const* grad, int* status, bool tridiag_only, double* tau_out = nullptr,
                        double* const* refl_out = nullptr, bool host_in = false,
-                       double* const* grad_host = nullptr) {
+                       double* const* grad_host = nullptr, bool any_order = false) {
   cudaStream_t st = P->h->stream;
   CK(cudaMemsetAsync(P->d_counters, 0, 2 * sizeof(unsigned) * std::max<size_t>(P->buckets.size(), 1), st));
   for (size_t i = 0; i < P->buckets.size(); i++) {
@@ -751,6 +766,12 @@ static int run_buckets(skew_batch_plan_t P, const double* const* A, double* logp
     bp.refl_out = refl_out;
     bp.status = status;
     bp.host_in = host_in ? 1 : 0;
+    int grid = B.grid;
+    if (B.grid_wide > 0 && any_order) {
+      grid = B.grid_wide;
+      bp.nt = 512;
+      bp.split = B.begin;
+    }
     bp.grad_host = grad_host;
     // gradients of the global-memory matrices: the reduction alone, then the products of all
     // of them on the tensor cores
@@ -761,7 +782,7 @@ static int run_buckets(skew_batch_plan_t P, const double* const* A, double* logp
       bp.tau_out = P->pg_tau;
       bp.refl_out = P->pg_refl;
     }
-    CK(launch_batch_pf(bp, B.grid, st, tridiag_only));
+    CK(launch_batch_pf(bp, grid, st, tridiag_only));
     if (pg) {
       PfGrad g;
       g.order = P->d_order + B.begin;
@@ -1179,7 +1200,8 @@ static int eigen_run(skew_batch_plan_t P, const double* const* A, double* const*
   if (ev_in)
     CK(launch_copy_ev(ev_in, P->d_n, P->d_ev_off, (int)P->count, P->d_ev, st));
   else
-    s = run_buckets(P, A, nullptr, nullptr, nullptr, nullptr, true, P->e_tau, P->e_p_refl);
+    s = run_buckets(P, A, nullptr, nullptr, nullptr, nullptr, true, P->e_tau, P->e_p_refl, false, nullptr,
+                    chain_nmax < P->nmax);
   if (s) return s;
   EigenBatch E;
   E.count = (int32_t)P->count;
