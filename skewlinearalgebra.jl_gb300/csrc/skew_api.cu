@@ -704,8 +704,14 @@ int skew_batch_plan_destroy(skew_batch_plan_t P) {
 // fused kernel, which needs none.
 static int pfgrad_ws(skew_batch_plan_t P) {
   if (P->pg_state != 0) return SKEW_OK;
-  P->pg_state = -1;
   cudaStream_t st = P->h->stream;
+  // inside a caller's capture nothing is allocated: the fused kernel this time
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
+    (void)cudaGetLastError();
+    return SKEW_OK;
+  }
+  P->pg_state = -1;
   std::vector<int32_t> order(P->count);
   std::iota(order.begin(), order.end(), 0);
   std::stable_sort(order.begin(), order.end(), [&](int32_t a, int32_t c) { return P->n_host[a] > P->n_host[c]; });
@@ -719,13 +725,20 @@ static int pfgrad_ws(skew_batch_plan_t P) {
     }
   }
   if (total == 0) return SKEW_OK;
-  if (cudaMallocAsync(&P->pg_ws, sizeof(double) * total, st) != cudaSuccess) {
+  auto alloc = [&](auto** p, size_t bytes) {
+    if (cudaMallocAsync(p, bytes, st) == cudaSuccess) return true;
     (void)cudaGetLastError();
+    *p = nullptr;
+    return false;
+  };
+  if (!alloc(&P->pg_ws, sizeof(double) * total) || !alloc(&P->pg_tau, sizeof(double) * P->ev_total) ||
+      !alloc(&P->pg_refl, sizeof(double*) * P->count)) {
+    if (P->pg_ws) CK(cudaFreeAsync(P->pg_ws, st));
+    if (P->pg_tau) CK(cudaFreeAsync(P->pg_tau, st));
     P->pg_ws = nullptr;
+    P->pg_tau = nullptr;
     return SKEW_OK;
   }
-  CK(cudaMallocAsync(&P->pg_tau, sizeof(double) * P->ev_total, st));
-  CK(cudaMallocAsync(&P->pg_refl, sizeof(double*) * P->count, st));
   std::vector<double*> ptr(P->count, nullptr);
   for (int64_t b = 0; b < P->count; b++)
     if (off[b] != SIZE_MAX) ptr[b] = P->pg_ws + off[b];
