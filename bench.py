@@ -34,10 +34,9 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 sys.path.insert(0, os.path.join(ROOT, "skewlinearalgebra.jl_gb300"))
 
-# dram__bytes_read.sum + dram__bytes_write.sum over the four batch_kernel launches of one
-# step of the default workload (4096 matrices, even n in [16, 256]), from one ncu capture
-# of the timed step (-s 12 -c 4)
-STEP_DRAM_BYTES = 20_753_729_792
+# DRAM bytes of one step of the default workload: not captured since the gradients of the
+# larger matrices left batch_kernel (20.75 GB per step before)
+STEP_DRAM_BYTES = None
 METRIC = "batched log|Pf|+grad matrices/s & n=8192 hessenberg GFLOP/s vs plain GPU, err≤1e-11"
 UNIT = "matrices/s"
 COUNT = 4096
@@ -420,7 +419,8 @@ def main():
     staged_sec = replicas.max_over_ranks(e0.elapsed_time(e1) / 1e3, dist, "cuda")
     staged_value = replicas.weak_scaling_throughput(count, world, e2e_steps, staged_sec)
 
-    # roofline of the dominant kernel (batch_kernel: every launch of a step)
+    # roofline of a step: batch_kernel (reductions, gradients up to the shared-memory sizes) on
+    # the FP64 pipe, the other gradients' products on the tensor cores
     flops = float(flops_per_matrix(sizes).sum())
     achieved_tflops = flops / (ms_dev / args.steps / 1e3) / 1e12
 
@@ -538,8 +538,7 @@ def main():
                                       "around skew_batch_logabspf_d on one stream"}},
             "roofline": {"bound": "fp64", "achieved": achieved_tflops, "peak": fp64_peak, "unit": "TFLOP/s",
                          "frac": achieved_tflops / fp64_peak, "traffic": STEP_DRAM_BYTES if (count, args.nmin, args.nmax) == (COUNT, NMIN, NMAX) else None,
-                         "traffic_unit": "bytes per step (DRAM read + write of the step's batch_kernel "
-                                         "launches, one ncu capture of the default workload)",
+                         "traffic_unit": "bytes per step (DRAM read + write)",
                          "algorithmic_bytes_per_step": int(2 * total * 8),
                          "peak_source": "FP64 DFMA peak measured live by skew_measure_fp64_peak "
                                         "(MEASURED_PEAKS.json has no FP64 figure)",
@@ -1133,10 +1132,11 @@ def leg_exp_adjoint(fp64_peak, steps, count=512):
 
 
 def _launches_per_call(sizes):
-    """batch_kernel launches of one batched call: one per size bucket of
+    """Kernel launches of one batched log|Pf| + gradient call: a batch_kernel per size bucket of
     skew_batch_plan_create (tuning key bucket_edges), the buckets whose working copies
     live in global memory (above batch_smem_nmax) merged into one launch when
-    batch_merge_global is set."""
+    batch_merge_global is set, and after each of those the gradients' products: 8 launches
+    and 2 per panel of 128 reflectors."""
     import skewgpu
 
     edges = skewgpu.tuning_get("bucket_edges")
@@ -1147,8 +1147,10 @@ def _launches_per_call(sizes):
         e = next((e for e in edges if n <= e), 1 << 30)
         buckets[e] = max(buckets[e], int(n))
     smem = sum(1 for e, nmax in buckets.items() if nmax <= smem_nmax)
-    glob = len(buckets) - smem
-    return smem + (min(glob, 1) if merge else glob)
+    glob = [nmax for nmax in buckets.values() if nmax > smem_nmax]
+    if merge and glob:
+        glob = [max(glob)]
+    return smem + sum(1 + 8 + 2 * -(-(nmax - 2) // 128) for nmax in glob)
 
 
 if __name__ == "__main__":

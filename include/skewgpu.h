@@ -97,7 +97,7 @@ SKEW_API int skew_logabspf_grad_d(skew_handle_t h, double* A, int64_t n, int64_t
 /* LA.eigvals!(A::SkewHermitian{Float64})  eigen.jl:2-6 -> skeweigvals! :49-55.
  * vals_im[n] = imaginary parts of the eigenvalues (eigenvalue k is i*vals_im[k]).
  * n <= 1024: in the reference's order, the deflation order of skewtrieigvals!
- * (skeweigen.jl:105-156), run on one GPU thread after the reduction; info receives
+ * (skeweigen.jl:105-156), run on four lanes after the reduction; info receives
  * SKEW_OK, SKEW_FALLBACK_USED (the shifts stagnated and the values come from the
  * reference's fallback, sorted descending, skeweigen.jl:132-137) or
  * SKEW_NO_CONVERGENCE (skeweigen.jl:154).  n > 1024: sorted descending by bisection

@@ -3,21 +3,22 @@
 //
 // Pipeline (after the batched reduction of skew_batch.cu has left the
 // reflectors, tau and ev of every matrix in the plan's workspace):
-//   chain   one thread per matrix runs the implicit QR of skewtrieigen_divided!
+//   chain   four lanes per matrix run the implicit QR of skewtrieigen_divided!
 //           (skeweigen.jl:322-377): same tolerance (10 eps), shift, deflation
 //           order, the |ev[n-1] - mem| < tol deflation (:355) and the stagnation
 //           counter.  The iteration on ev never depends on the eigenvectors, so
 //           every Givens rotation is logged instead of applied.
-//   vectors one CTA per matrix replays the log on Qodd / Qeven (lanes are rows:
-//           every row is rotated independently), applies the odd-size rotations
+//   vectors a warp per 32 rows of Qodd or Qeven replays the log (every row is rotated
+//           independently); then one CTA per matrix applies the odd-size rotations
 //           of reducetozero (getoddvectors, :49-62) and assembles the real and
 //           imaginary eigenvector parts with the reference's +-1/sqrt(2) pairing
 //           (:378-449).  If the QR stagnated, the eigenvectors of the symmetric
-//           tridiagonal SymTridiagonal(0, ev) come from a cyclic Jacobi solver
+//           tridiagonal SymTridiagonal(0, ev) come from bisection and twisted vectors
 //           in the same CTA and are laid out as skewtrieigen_backup! does
 //           (:470-489).
-//   back    V <- Q V for both parts (eigen.jl:85-89) by compact-WY blocks of 8
-//           reflectors: Y = V_b^T X, Z = T_b Y, X -= V_b Z.
+//   back    V <- Q V for both parts (eigen.jl:85-89) by compact-WY panels of 128
+//           reflectors on the tensor cores (skew_back.cuh); small matrices by blocks of 8:
+//           Y = V_b^T X, Z = T_b Y, X -= V_b Z.
 //   exp     E = Qr P^T + Qi R^T with P = Qr C + Qi S, R = Qi C - Qr S
 //           (C, S = cos, sin of the eigenvalues; exp.jl:3-35 reassociated).
 //   cis     V diag(exp(-Im lambda)) V^H (exp.jl:99-110), two real products.
