@@ -1412,7 +1412,7 @@ static int eigen_large(skew_handle_t h, double* A, int64_t n, int64_t lda, doubl
                        int64_t ldv, int* info) {
   if (lda < n || ldv < n || n > (1LL << 15)) return n > (1LL << 15) ? SKEW_UNSUPPORTED : SKEW_BAD_ARG;
   const size_t wsd = reduce_ws_doubles(n);
-  const size_t lwsd = large_eigen_ws_doubles((int)n), auxd = large_eigen_aux_doubles((int)n);
+  const size_t lwsd = large_vectors_ws_doubles((int)n), auxd = large_eigen_aux_doubles((int)n);
   const size_t extra = 2 * (size_t)n + 8 + lwsd + auxd + 1;
   int st = ensure_ws(h, sizeof(double) * (wsd + extra));
   if (st) return st;

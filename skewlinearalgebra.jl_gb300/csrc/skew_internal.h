@@ -206,10 +206,13 @@ cudaError_t zfunc_from_eigen(int mode, int func, int n, const double* vals_im, c
 size_t large_eigen_ws_doubles(int n);
 cudaError_t symtri_vectors(const double* dg, const double* e, int n, const double* mu, const double* bp, double* Y,
                            double* ws, int batch, cudaStream_t st);
+// ws: the twisted kernels' workspace (large_eigen_ws_doubles) and, with A, the
+// back-transformation's in the same place (large_vectors_ws_doubles).
 // gate: a device int of scratch; aux: large_eigen_aux_doubles(n) doubles of scratch.
 // A tridiagonal that splits exactly into more odd-size blocks than n mod 2 (several
 // zero eigenvalues) is solved in full mode, as the reference's fallback does.
 size_t large_eigen_aux_doubles(int n);
+size_t large_vectors_ws_doubles(int n);
 cudaError_t large_eigen_vectors(const double* A, int64_t lda, int n, const double* tau, const double* ev,
                                 const double* vals, const double* bp, double* Vr, double* Vi, int64_t ldv, double* ws,
                                 int* gate, double* aux, cudaStream_t st);

@@ -597,7 +597,9 @@ __global__ void __launch_bounds__(LA_NT) tdvec_write_fallback_batch_kernel(Tdvec
 
 // Strips of 32 columns per CTA walking all panels on the FP64 pipe took 43.5 ms at
 // n = 2048; panel by panel on the tensor cores 2.8 ms.  The vectors are in Vr and Vi, so
-// the workspace of the twisted kernels (3 n KP doubles of the full mode) is free.
+// the workspace of the twisted kernels is free; W is split as far as their 3 n KP doubles
+// go.  Unsplit, the 2 n columns of the full mode need more than those at n = 96,
+// 109 .. 128 and 131 .. 192: large_vectors_ws_doubles covers both.
 static cudaError_t back_transform(const double* A, int64_t lda, const double* tau, const TdvecLayout& L, double* Vr,
                                   double* Vi, int64_t ldv, int cr0, int ci0, double* ws, cudaStream_t st) {
   const int n = L.n;
@@ -622,13 +624,17 @@ static cudaError_t back_transform(const double* A, int64_t lda, const double* ta
   const size_t room = 3 * (size_t)n * ((n + 31) / 32 * 32);
   int splits = back_splits(cols, 1, sms);
   while (splits > 1 && back_ws_doubles<false>(n, n - 2, cols, splits) > room) splits /= 2;
+  if (back_ws_doubles<false>(n, n - 2, cols, splits) > large_vectors_ws_doubles(n)) return cudaErrorInvalidValue;
   back_ws_set(S.B, ws, cols, splits);
   return back_transform_oz<false>(S, 1, n, n - 2, cols, splits, st);
 }
 
 size_t large_eigen_aux_doubles(int n) { return (size_t)n + 8; }
+size_t large_vectors_ws_doubles(int n) {
+  return std::max(large_eigen_ws_doubles(n), n > 2 ? back_ws_doubles<false>(n, n - 2, 2 * n, 1) : 0);
+}
 
-// gate (device int) and aux (large_eigen_aux_doubles(n)) are scratch of the caller.
+// ws: large_vectors_ws_doubles(n), or large_eigen_ws_doubles(n) without A.  gate (device int) and aux (large_eigen_aux_doubles(n)) are scratch of the caller.
 cudaError_t large_eigen_vectors(const double* A, int64_t lda, int n, const double* tau, const double* ev,
                                 const double* vals, const double* bp, double* Vr, double* Vi, int64_t ldv, double* ws,
                                 int* gate, double* aux, cudaStream_t st) {
