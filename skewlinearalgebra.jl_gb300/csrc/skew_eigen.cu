@@ -1005,7 +1005,7 @@ cudaError_t launch_eigen_back(const EigenBatch& E, int grid, int nmax, cudaStrea
 // from phi0 to phi1 (m the mean, delta half the difference): -mu_a -> -mu_b for P,
 // mu_a -> -mu_b for N.  A 1 x 2, 2 x 1 or 1 x 1 block (zero eigenvalue) takes the
 // same with mu = 0.  Four real n x n products instead of the twelve of the complex
-// form.  With tol = 64 eps max|mu|, the columns with mu > tol give two Q columns,
+// form.  With tol = 64 eps max|mu| (1e-307 for a zero matrix), the columns with mu > tol give two Q columns,
 // |mu| <= tol one and mu < -tol none.  A zero eigenvalue that a full tridiagonal
 // solve returns as a few ulps (several odd blocks, the Jacobi fallback) is then a
 // real single column, not half of a pair; its function value is f(0) (singular for
@@ -1058,7 +1058,8 @@ __global__ void __launch_bounds__(SB_NT) schur_scan_kernel(EigenBatch E) {
   __syncthreads();
   mx = 0.0;
   for (int q = 0; q < SB_NT / 32; q++) mx = fmax(mx, red[q]);
-  const double tol = 64.0 * 2.220446049250313e-16 * mx;
+  // the bisection ends within 8.9e-308 of a zero eigenvalue
+  const double tol = fmax(64.0 * 2.220446049250313e-16 * mx, 1e-307);
   long long base = 0, nblk = 0;
   for (int j0 = 0; j0 < n; j0 += SB_NT) {
     const int j = j0 + tid;
