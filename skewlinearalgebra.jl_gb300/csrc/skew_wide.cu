@@ -786,7 +786,8 @@ __global__ void __launch_bounds__(256) fxp_exps_kernel(const double* __restrict_
   if ((threadIdx.x & 31) == 0) atomicMax(w.sync + 2, (unsigned)b);
 }
 
-// C = [V 2^k | W] [W | -V 2^k]^T = 2^k (V W^T - W V^T), k bringing V to the size of W.
+// C = [V | W 2^-k] [W 2^-k | -V]^T = 2^-k (V W^T - W V^T), 2^k the size of W: both factors
+// near 1, so C stays in range for any A (V scaled to W instead would square A's scale).
 struct FxpUpdate {
   double* A;
   int64_t lda;
@@ -801,7 +802,7 @@ struct FxpUpdate {
   __device__ int exponent(int r) const {
     const int a = w.ev[q + r], b = w.ew[q + r];
     if (a == 2047 || b == 2047) return 2047;
-    return min(2046, max(max(a + k, b), 1));
+    return min(2046, max(max(a, b - k), 1));
   }
   __device__ int expA(int i) const { return exponent(i); }
   __device__ int expB(int j) const { return exponent(j); }
@@ -814,14 +815,14 @@ struct FxpUpdate {
     for (int u = 0; u < NV; u++) {
       double x = 0.0;
       if (l0 + u < nbp) x = vside ? A[q + r + (int64_t)(p + l0 + u) * lda] : w.W[(size_t)(l0 + u) * n + q + r];
-      if (vside) x = oz_ldexp(x, k);
+      if (!vside) x = oz_ldexp(x, -k);
       v[u] = (vside && !left) ? neg(x) : x;
     }
   }
   __device__ void loadA(int i, int s, int kk, double (&v)[8]) const { load<8>(i, s * OZ_K + kk, true, v); }
   __device__ void loadB(int j, int s, int kk, double (&v)[4]) const { load<4>(j, s * OZ_K + kk, false, v); }
   __device__ void store(int i, int j, double x) const {
-    if (i > j) A[q + i + (int64_t)(q + j) * lda] += oz_ldexp(x, -k);
+    if (i > j) A[q + i + (int64_t)(q + j) * lda] += oz_ldexp(x, k);
   }
   __device__ void timeout() const { w.sync[1] = 1u; }
 };

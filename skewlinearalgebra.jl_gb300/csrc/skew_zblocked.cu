@@ -633,8 +633,9 @@ __global__ void __launch_bounds__(256) zp_exps_kernel(ZPersistParams P) {
   }
 }
 
-// Real rows 2 r, 2 r + 1 of the result (re, im of row r: neighbours in memory), 2^k (V W^H -
-// W V^H) as four buffers of at most 32 terms, k bringing V to the size of W:
+// Real rows 2 r, 2 r + 1 of the result (re, im of row r: neighbours in memory), 2^-k (V W^H -
+// W V^H) as four buffers of at most 32 terms, W scaled by 2^-k to the size of V, so that the
+// products stay in range for any A:
 //   re: vr wr' + vi wi' + wr (-vr') + wi (-vi'),   im: vi wr' + (-vr) wi' + wi (-vr') + (-wr) (-vi').
 struct ZpUpdate {
   ZPersistParams P;
@@ -647,7 +648,7 @@ struct ZpUpdate {
   __device__ int exponent(int r) const {
     const int a = P.ea[q + r], b = P.ew[q + r];
     if (a == 2047 || b == 2047) return 2047;
-    return min(2046, max(max(a + k, b), 1));
+    return min(2046, max(max(a, b - k), 1));
   }
   __device__ int expA(int i) const { return exponent(i >> 1); }
   __device__ int expB(int j) const { return exponent(j); }
@@ -659,7 +660,7 @@ struct ZpUpdate {
 #pragma unroll
     for (int u = 0; u < NV; u++) {
       double x = (l0 + u < P.nbp) ? src[u * ld] : 0.0;
-      if (vside) x = oz_ldexp(x, k);
+      if (!vside) x = oz_ldexp(x, -k);
       v[u] = minus ? neg(x) : x;
     }
   }
@@ -671,7 +672,7 @@ struct ZpUpdate {
     const int r = i >> 1, part = i & 1;
     if (r < j || (r == j && part == 0)) return;  // the diagonal receives the imaginary part only
     double* a = reinterpret_cast<double*>(P.A + q + r + (int64_t)(q + j) * P.lda) + part;
-    const double y = *a + oz_ldexp(x, -k);
+    const double y = *a + oz_ldexp(x, k);
     *a = y;
     if (r > j) reinterpret_cast<double*>(P.A + q + j + (int64_t)(q + r) * P.lda)[part] = part ? y : neg(y);
   }
