@@ -90,12 +90,12 @@ __device__ __forceinline__ double oz_double(long long v, int e) {
   return __longlong_as_double((long long)(bits | ((unsigned long long)(v < 0) << 63)));
 }
 
-// x 2^k: the exponent field where it stays normal, else by multiplication (out of line: as
-// a select it would put FP64 instructions on every entry)
+// x 2^k: the exponent field where x is finite and stays normal, else by multiplication (out
+// of line: as a select it would put FP64 instructions on every entry)
 static __device__ __noinline__ double oz_ldexp_edge(double x, int k) { return scalbn(x, k); }
 __device__ __forceinline__ double oz_ldexp(double x, int k) {
   const int h = __double2hiint(x), e = (h >> 20) & 0x7ff;
-  if (e != 0 && (unsigned)(e + k - 1) < 2045u) return __hiloint2double(h + (k << 20), __double2loint(x));
+  if ((unsigned)(e - 1) < 2046u && (unsigned)(e + k - 1) < 2045u) return __hiloint2double(h + (k << 20), __double2loint(x));
   return x == 0.0 ? x : oz_ldexp_edge(x, k);
 }
 
