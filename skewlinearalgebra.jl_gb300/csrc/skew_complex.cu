@@ -114,6 +114,7 @@ __global__ void __launch_bounds__(ZNT) zhess_cta_kernel(ZHessParams P) {
   zc* W = reinterpret_cast<zc*>(P.W) + (int64_t)b * P.stride;
   zc* tau = reinterpret_cast<zc*>(P.tau) + (int64_t)b * n;
   double* ev = P.ev + (int64_t)b * n;
+  if (CS > 1) cl.sync();  // all CTAs run before the first write into another's shared memory
   for (int c = 0; c + 1 < n; c++) {
     const int m = n - c - 1;
     zc* x = W + (c + 1) + (int64_t)c * ld;
