@@ -116,7 +116,8 @@ __device__ __forceinline__ void oz_mma(uint32_t d, uint64_t a, uint64_t b, uint3
       : "memory");
 }
 
-// Bounded wait for a phase of an mbarrier.
+// Bounded wait for a phase of an mbarrier, by a whole warp (the lanes agree on the outcome:
+// warp-wide instructions follow).
 __device__ __forceinline__ bool oz_wait(uint32_t bar, uint32_t parity) {
   for (int t = 0; t < OZ_POLLS; t++) {
     uint32_t done;
@@ -125,7 +126,7 @@ __device__ __forceinline__ bool oz_wait(uint32_t bar, uint32_t parity) {
         : "=r"(done)
         : "r"(bar), "r"(parity)
         : "memory");
-    if (done) return true;
+    if (__all_sync(0xffffffffu, done)) return true;
   }
   return false;
 }
@@ -317,7 +318,12 @@ __device__ __forceinline__ void oz_tile(const Prob& P, int i0, int j0, unsigned 
     ok = oz_wait(oz_smem(bars + w), (uses[w] - 1) & 1);
     if (ok) drain();
   }
-  ok = __syncthreads_and(ok);
+  if (!__syncthreads_and(ok)) {  // a wait gave up: what was issued ends before its memory is given back
+    ok = false;
+    for (int w = 0; w < 2; w++)
+      if (uses[w] > 0) oz_wait(oz_smem(bars + w), (uses[w] - 1) & 1);
+    __syncthreads();
+  }
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
   if (!ok) {
     if (tid == 0) P.timeout();
