@@ -367,7 +367,8 @@ SKEW_API int skew_tridiag_svd_z(skew_handle_t h, const double* ev, const double*
  * complex panel width, 4..32), pfz_cta_max, pfz_nt, pfz_ctas, and the limits
  * wait_polls (grid-barrier polls before SKEW_TIMEOUT; 0: the default, seconds),
  * wait_skip_cta (>= 0: that CTA of a cooperative kernel skips its arrivals, so the
- * bounded waits run out: a test of the timeout path; -1: off) and qr_max_iter (QR
+ * bounded waits run out, and its tiles of a single matrix's or a complex
+ * back-transformation: a test of the timeout path; -1: off) and qr_max_iter (QR
  * sweeps before SKEW_NO_CONVERGENCE; 0: the reference's 30 n, skeweigen.jl:115).
  * Batch plans take the bucket keys when they are created.  No reference counterpart.
  * ------------------------------------------------------------------------- */

@@ -1427,7 +1427,8 @@ static int eigen_large(skew_handle_t h, double* A, int64_t n, int64_t lda, doubl
   st = blocked(h, A, n, lda, tau, ev, info, extra, nullptr);
   if (st) return st;
   CK(launch_tridiag_bisect(ev, (int)n, vals_im, bp, h->stream));
-  CK(large_eigen_vectors(A, lda, (int)n, tau, ev, vals_im, bp, Vr, Vi, ldv, lws, gate, aux, h->stream));
+  CK(large_eigen_vectors(A, lda, (int)n, tau, ev, vals_im, bp, Vr, Vi, ldv, lws, gate, aux, info,
+                         h->tune.wait_skip_cta, h->stream));
   return SKEW_OK;
 }
 
@@ -1616,7 +1617,7 @@ int skew_eigvals_z(skew_handle_t h, double* A, int64_t n, int64_t lda, double* v
   if (st) return st;
   st = zreduce(h, A, n, lda, 1, L.tau, L.ev, L.dvim, L.zws, info);
   if (st) return st;
-  CK(zeigen_from_tridiag(A, lda, (int)n, L.tau, L.ev, L.dvim, vals_im, nullptr, 0, L.ews, 1, h->stream));
+  CK(zeigen_from_tridiag(A, lda, (int)n, L.tau, L.ev, L.dvim, vals_im, nullptr, 0, L.ews, 1, info, -1, h->stream));
   return SKEW_OK;
 }
 
@@ -1632,7 +1633,8 @@ int skew_eigen_z(skew_handle_t h, double* A, int64_t n, int64_t lda, double* val
   if (st) return st;
   st = zreduce(h, A, n, lda, 1, L.tau, L.ev, L.dvim, L.zws, info);
   if (st) return st;
-  CK(zeigen_from_tridiag(A, lda, (int)n, L.tau, L.ev, L.dvim, vals_im, V, ldv, L.ews, 1, h->stream));
+  CK(zeigen_from_tridiag(A, lda, (int)n, L.tau, L.ev, L.dvim, vals_im, V, ldv, L.ews, 1, info, h->tune.wait_skip_cta,
+                         h->stream));
   return SKEW_OK;
 }
 
@@ -1648,7 +1650,8 @@ static int zfunc(skew_handle_t h, double* A, int64_t n, int64_t lda, const doubl
   if (st) return st;
   st = zreduce(h, A, n, lda, 1, L.tau, L.ev, L.dvim, L.zws, info);
   if (st) return st;
-  CK(zeigen_from_tridiag(A, lda, (int)n, L.tau, L.ev, L.dvim, L.vals, L.V, n, L.ews, 1, h->stream));
+  CK(zeigen_from_tridiag(A, lda, (int)n, L.tau, L.ev, L.dvim, L.vals, L.V, n, L.ews, 1, info, h->tune.wait_skip_cta,
+                         h->stream));
   CK(zfunc_from_eigen(mode, func, (int)n, L.vals, L.V, n, C, n, O, ldo, L.fws, 1, info, h->stream));
   return SKEW_OK;
 }
@@ -1679,7 +1682,8 @@ static int zbatch(skew_handle_t h, const double* A, int64_t n, int64_t count, do
   if (st) return st;
   double* vv = mode < 0 ? vals_im : L.vals;
   double* VV = mode < 0 ? V : L.V;
-  CK(zeigen_from_tridiag(L.W, n, (int)n, L.tau, L.ev, L.dvim, vv, VV, n, L.ews, (int)count, h->stream));
+  CK(zeigen_from_tridiag(L.W, n, (int)n, L.tau, L.ev, L.dvim, vv, VV, n, L.ews, (int)count, status,
+                         h->tune.wait_skip_cta, h->stream));
   if (mode >= 0) CK(zfunc_from_eigen(mode, func, (int)n, vv, VV, n, C, n, O, n, L.fws, (int)count, status, h->stream));
   return SKEW_OK;
 }
@@ -2002,7 +2006,7 @@ int skew_tridiag_eigen_d(skew_handle_t h, const double* ev, int64_t n, double* v
     if (info) CK(cudaMemsetAsync(info, 0, sizeof(int), h->stream));
     CK(launch_tridiag_bisect(ev, (int)n, vals_im, bp, h->stream));
     CK(large_eigen_vectors(nullptr, 0, (int)n, nullptr, ev, vals_im, bp, Vr, Vi, ldv, bp + 8, (int*)(aux + auxd),
-                           aux, h->stream));
+                           aux, info, -1, h->stream));
     return SKEW_OK;
   }
   if (ldv != n) return SKEW_UNSUPPORTED;

@@ -42,7 +42,8 @@ struct BackTask {
   double *t, *vt, *w;     // T: panels of ldt x ldt; VT: R n x nref; W: R ldt x columns (x splits)
   int *et, *evt, *ex;     // exponents: T's columns, VT's rows per panel, X's columns
   int identity;           // X starts as the identity: a panel from column c0 leaves columns 0 .. c0 alone
-  int* status;
+  int* status;            // SKEW_TIMEOUT if a bounded wait gave up (or null)
+  int skip_cta = -1;      // >= 0: this CTA of each X <- X - VT W counts as given up (a test of the status)
   __host__ __device__ int ldt() const { return nref < BK<CX>::PB ? nref : BK<CX>::PB; }
   __host__ __device__ int panels() const { return (nref + BK<CX>::PB - 1) / BK<CX>::PB; }
   __device__ int cols() const { return nc[0] + nc[1]; }
@@ -406,6 +407,10 @@ __global__ void __launch_bounds__(OZ_NT, 1) back_x_kernel(Src S, int step, int r
   P.nb = min(BK<CX>::PB, P.B.nref - P.c0);
   const int i0 = (int)(blockIdx.x % rt) * OZ_M, j0 = (int)(blockIdx.x / rt) * OZ_N;
   if (i0 >= P.rows() || j0 >= P.cols() || (P.B.identity && j0 + OZ_N - 1 <= P.c0)) return;
+  if ((int)blockIdx.x == P.B.skip_cta) {
+    if (threadIdx.x == 0) P.timeout();
+    return;
+  }
   oz_tile(P, i0, j0, oz_buf);
 }
 

@@ -721,6 +721,7 @@ struct ZBack {
     T.et += 2 * o;
     T.evt += 2 * o;
     T.ex += 2 * o;
+    if (T.status) T.status += b;
     return true;
   }
 };
@@ -750,7 +751,7 @@ size_t zeigen_ws_doubles(int n, int batch) {
 // V != null, the eigenvectors V (ldv*n apart).
 cudaError_t zeigen_from_tridiag(const double* Ad, int64_t lda, int n, const double* taud, const double* ev,
                                 const double* dvim, double* vals_im, double* Vd, int64_t ldv, double* ws, int batch,
-                                cudaStream_t st) {
+                                int* status, int skip_cta, cudaStream_t st) {
   const size_t B = (size_t)batch;
   double* dg = ws;
   double* off = dg + seg(B * n);
@@ -783,7 +784,8 @@ cudaError_t zeigen_from_tridiag(const double* Ad, int64_t lda, int n, const doub
   S.B.nc[0] = n;
   S.B.nc[1] = 0;
   S.B.identity = 0;
-  S.B.status = nullptr;
+  S.B.status = status;
+  S.B.skip_cta = skip_cta;
   int splits = 1;
   if (nextra) {
     S.stride = seg(back_ws_doubles<true>(n, n - 1, n, 1));

@@ -67,7 +67,8 @@ struct Tuning {
   int pfz_ctas;                  // grid of the cooperative Pfaffian (0: chosen by n)
   // bounded waits and iteration limits
   long long wait_polls;          // grid-barrier polls before SKEW_TIMEOUT (0: the kernel's default)
-  int wait_skip_cta;             // >= 0: this CTA skips its arrivals, so the barrier waits run out
+  int wait_skip_cta;             // >= 0: this CTA skips its arrivals, so the barrier waits run out, and its
+                                 // tiles of a back-transformation
   int qr_max_iter;               // > 0: QR sweeps before SKEW_NO_CONVERGENCE (0: 30 n, the reference's)
 };
 void tuning_defaults(Tuning* T);
@@ -186,11 +187,13 @@ cudaError_t zhess_persistent(double* A, int64_t lda, int n, double* tau, double*
 cudaError_t zhess_large(double* A, int64_t lda, int n, double* tau, double* ev, double* dvim, double* ws,
                         cudaStream_t st);
 // complex eigen from `batch` reduced matrices of size n (arrays per matrix: A lda*n,
-// tau/ev/dvim/vals n, V ldv*n apart); values descending (-mu, mu ascending), vectors Q D Y
+// tau/ev/dvim/vals n, V ldv*n apart); values descending (-mu, mu ascending), vectors Q D Y.
+// status (one per problem, or null) <- SKEW_TIMEOUT if a bounded wait gave up; skip_cta:
+// Tuning::wait_skip_cta
 size_t zeigen_ws_doubles(int n, int batch);
 cudaError_t zeigen_from_tridiag(const double* A, int64_t lda, int n, const double* tau, const double* ev,
                                 const double* dvim, double* vals_im, double* V, int64_t ldv, double* ws, int batch,
-                                cudaStream_t st);
+                                int* status, int skip_cta, cudaStream_t st);
 // mode 0: O = V f(i mu) V^H for the matrix function `func` (skew_func_t), projected on
 // the Hermitian / skew-Hermitian part where the function's result has that symmetry;
 // mode 1: the adjoint of exp, O = V (conj(Phi) o (V^H C V)) V^H.  `batch` problems with
@@ -208,6 +211,7 @@ cudaError_t symtri_vectors(const double* dg, const double* e, int n, const doubl
                            double* ws, int batch, cudaStream_t st);
 // ws: the twisted kernels' workspace (large_eigen_ws_doubles) and, with A, the
 // back-transformation's in the same place (large_vectors_ws_doubles).
+// info (or null) <- SKEW_TIMEOUT if a bounded wait gave up; skip_cta: Tuning::wait_skip_cta.
 // gate: a device int of scratch; aux: large_eigen_aux_doubles(n) doubles of scratch.
 // A tridiagonal that splits exactly into more odd-size blocks than n mod 2 (several
 // zero eigenvalues) is solved in full mode, as the reference's fallback does.
@@ -215,7 +219,7 @@ size_t large_eigen_aux_doubles(int n);
 size_t large_vectors_ws_doubles(int n);
 cudaError_t large_eigen_vectors(const double* A, int64_t lda, int n, const double* tau, const double* ev,
                                 const double* vals, const double* bp, double* Vr, double* Vi, int64_t ldv, double* ws,
-                                int* gate, double* aux, cudaStream_t st);
+                                int* gate, double* aux, int* info, int skip_cta, cudaStream_t st);
 
 // Eigenvectors / exp / cis / exp adjoint for batches of real skew matrices (skew_eigen.cu).
 // Leading dimensions of every per-matrix n x n buffer are n.

@@ -601,7 +601,8 @@ __global__ void __launch_bounds__(LA_NT) tdvec_write_fallback_batch_kernel(Tdvec
 // go.  Unsplit, the 2 n columns of the full mode need more than those at n = 96,
 // 109 .. 128 and 131 .. 192: large_vectors_ws_doubles covers both.
 static cudaError_t back_transform(const double* A, int64_t lda, const double* tau, const TdvecLayout& L, double* Vr,
-                                  double* Vi, int64_t ldv, int cr0, int ci0, double* ws, cudaStream_t st) {
+                                  double* Vi, int64_t ldv, int cr0, int ci0, double* ws, int* info, int skip_cta,
+                                  cudaStream_t st) {
   const int n = L.n;
   int dev = 0, sms = 148;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -617,7 +618,8 @@ static cudaError_t back_transform(const double* A, int64_t lda, const double* ta
   S.B.nc[0] = n - cr0;
   S.B.nc[1] = n - ci0;
   S.B.identity = 0;
-  S.B.status = nullptr;
+  S.B.status = info;
+  S.B.skip_cta = skip_cta;
   S.gate = L.gate;
   S.gate_on = L.gate_on;
   const int cols = S.B.nc[0] + S.B.nc[1];
@@ -637,7 +639,7 @@ size_t large_vectors_ws_doubles(int n) {
 // ws: large_vectors_ws_doubles(n), or large_eigen_ws_doubles(n) without A.  gate (device int) and aux (large_eigen_aux_doubles(n)) are scratch of the caller.
 cudaError_t large_eigen_vectors(const double* A, int64_t lda, int n, const double* tau, const double* ev,
                                 const double* vals, const double* bp, double* Vr, double* Vi, int64_t ldv, double* ws,
-                                int* gate, double* aux, cudaStream_t st) {
+                                int* gate, double* aux, int* info, int skip_cta, cudaStream_t st) {
   if (n < 3) return cudaErrorInvalidValue;
   double* mu = aux;
   double* bpf = aux + n;
@@ -657,7 +659,7 @@ cudaError_t large_eigen_vectors(const double* A, int64_t lda, int n, const doubl
   if (e != cudaSuccess) return e;
   if (A) {  // A == null: a tridiagonal input, Q = I
     // -sigma columns and the zero vector of Vr, -sigma columns of Vi
-    e = back_transform(A, lda, tau, L, Vr, Vi, ldv, L.h, L.h + (n & 1), ws, st);
+    e = back_transform(A, lda, tau, L, Vr, Vi, ldv, L.h, L.h + (n & 1), ws, info, skip_cta, st);
     if (e != cudaSuccess) return e;
   }
   mirror_kernel<<<dim3((n + 255) / 256, L.h + (n & 1)), 256, 0, st>>>(Vr, Vi, ldv, n, gate);
@@ -674,7 +676,7 @@ cudaError_t large_eigen_vectors(const double* A, int64_t lda, int n, const doubl
   tdvec_write_fallback_kernel<<<dim3(F.KP / 32, (n + RC - 1) / RC), LA_NT, 0, st>>>(F, X, Vr, Vi, ldv);
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  if (A) return back_transform(A, lda, tau, F, Vr, Vi, ldv, 0, 0, ws, st);
+  if (A) return back_transform(A, lda, tau, F, Vr, Vi, ldv, 0, 0, ws, info, skip_cta, st);
   return cudaSuccess;
 }
 

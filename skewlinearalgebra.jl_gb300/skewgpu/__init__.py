@@ -339,6 +339,8 @@ def _info_ok(info: torch.Tensor, where: str) -> int:
     st = int(info.item())
     if st == _lib.SKEW_NO_CONVERGENCE:
         raise RuntimeError("Maximum number of iterations reached, the algorithm didn't converge")
+    if st == _lib.SKEW_TIMEOUT:
+        raise SkewError(st, where)
     return st
 
 
@@ -486,7 +488,7 @@ def matrix_function(A, name: str):
         F = torch.zeros((n, n), dtype=torch.float64, device="cuda")
         check(_lib.load().skew_func_d(h, _ptr(S.data), n, n, f, _ptr(F), n, _ptr(info)), name)
         out = from_device(F)
-    if int(info.item()) == _lib.SKEW_SINGULAR:
+    if _info_ok(info, name) == _lib.SKEW_SINGULAR:
         raise ValueError(f"{name} of a singular matrix doesn't exist")
     return out
 
@@ -667,6 +669,7 @@ def eigen_complex(A):
     info = _info_tensor()
     h = handle().bind()
     check(_lib.load().skew_eigen_z(h, _ptr(W), n, n, _ptr(vals), _ptr(V), n, _ptr(info)), "eigen_complex")
+    _info_ok(info, "eigen_complex")
     return 1j * vals.cpu().numpy(), from_device_complex(V)
 
 
@@ -678,6 +681,7 @@ def exp_complex(A) -> np.ndarray:
     info = _info_tensor()
     h = handle().bind()
     check(_lib.load().skew_exp_z(h, _ptr(W), n, n, _ptr(E), n, _ptr(info)), "exp_complex")
+    _info_ok(info, "exp_complex")
     return from_device_complex(E)
 
 
@@ -695,6 +699,7 @@ def exp_complex_rrule(A):
         info = _info_tensor()
         h = handle().bind()
         check(_lib.load().skew_exp_vjp_z(h, _ptr(W), n, n, _ptr(Cd), _ptr(G), n, _ptr(info)), "exp_vjp_complex")
+        _info_ok(info, "exp_vjp_complex")
         return from_device_complex(G)
 
     return E, pullback
