@@ -439,7 +439,8 @@ cudaError_t launch_check_skew(const double* A, int64_t lda, int n, double* flag,
 }
 
 // log|Pf| and sign from ev and tau for one matrix (used after the blocked path).
-// notskew (nullable) is the flag of check_skew_kernel.
+// notskew (nullable) is the flag of check_skew_kernel.  A reduction that gave up (info,
+// written by every reduction before this) has no Pfaffian: NaN, and the status stays.
 __global__ void __launch_bounds__(256) pf_from_tridiag_kernel(const double* ev, const double* tau, int n,
                                                               double* logpf, double* sign, int* info,
                                                               const double* notskew) {
@@ -450,6 +451,10 @@ __global__ void __launch_bounds__(256) pf_from_tridiag_kernel(const double* ev, 
       *sign = nan("");
       if (info) *info = SKEW_NOT_SKEW;
     }
+    return;
+  }
+  if (info && *info == SKEW_TIMEOUT) {
+    if (threadIdx.x == 0) *logpf = *sign = nan("");
     return;
   }
   if (n & 1) {

@@ -227,8 +227,11 @@ def logabspfaffian_(A, check_skew: bool = False) -> Tuple[float, float]:
                                       int(check_skew), ctypes.c_void_p(p + 16)),
           "logabspfaffian")
     host = out.cpu().numpy()
-    if int(host[2:].view(np.int32)[0]) == _lib.SKEW_NOT_SKEW:
+    st = int(host[2:].view(np.int32)[0])
+    if st == _lib.SKEW_NOT_SKEW:
         raise ValueError("Pfaffian requires a skew-Hermitian matrix")
+    if st == _lib.SKEW_TIMEOUT:
+        raise SkewError(st, "logabspfaffian")
     return float(host[0]), float(host[1])
 
 

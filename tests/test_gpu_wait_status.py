@@ -52,3 +52,27 @@ def test_batched_complex_status(skewgpu):
     with skewgpu.tuned(wait_skip_cta=0):
         assert call() == [skewgpu._lib.SKEW_TIMEOUT] * count
     assert call() == [0] * count
+
+
+# the wide reduction, and without the cluster one the grid-wide one
+@pytest.mark.parametrize("n,keys", [(1100, {}), (512, dict(cluster_max_n=0))])
+def test_logabspf_keeps_the_reductions_timeout(skewgpu, n, keys):
+    A = _skewh(n, n).real / np.sqrt(n)
+    L, h = skewgpu._lib.load(), skewgpu.handle().bind()
+    out = torch.zeros(2, dtype=torch.float64, device="cuda")
+    info = torch.full((1,), -1, dtype=torch.int32, device="cuda")
+
+    def call():
+        W = skewgpu.to_device(A)
+        assert L.skew_logabspf_d(h, _p(W), n, n, _p(out), ctypes.c_void_p(out.data_ptr() + 8), 0, _p(info)) == 0
+        return int(info.item()), out.cpu().numpy()
+
+    ok, good = call()
+    with skewgpu.tuned(wait_polls=20000, wait_skip_cta=3, **keys):
+        bad, nans = call()
+        with pytest.raises(skewgpu.SkewError):
+            skewgpu.logabspfaffian(A)
+    again, after = call()
+    assert (ok, bad, again) == (0, skewgpu._lib.SKEW_TIMEOUT, 0)
+    assert np.isnan(nans).all()
+    np.testing.assert_array_equal(good, after)
