@@ -93,6 +93,7 @@ struct skew_batch_plan_st {
   int* e_fsel = nullptr;  // exp adjoint: per matrix, real Schur-basis (1) or complex (0) form
   int32_t* e_back_off = nullptr;  // back-transformation items before each matrix (processing order)
   int32_t back_items = 0;
+  int32_t back_large = 0;  // matrices from kBackOzMin on
   // one instantiated CUDA graph per batched operation, keyed on its arguments
   struct GraphSlot {
     bool valid = false;
@@ -1082,6 +1083,7 @@ static int eigen_ws(skew_batch_plan_t P) {
   std::stable_sort(ord.begin(), ord.end(), [&](int32_t a, int32_t c) { return P->n_host[a] > P->n_host[c]; });
   for (int64_t t = 0; t < count; t++) boff[t + 1] = boff[t] + back_items_of(P->n_host[ord[t]]);
   P->back_items = boff[count];
+  P->back_large = (int32_t)std::count_if(P->n_host.begin(), P->n_host.end(), [](int32_t n) { return n >= kBackOzMin; });
   ok &= cudaMemcpyAsync(P->e_back_off, boff.data(), sizeof(int32_t) * (count + 1), cudaMemcpyHostToDevice, st) ==
         cudaSuccess;
   if (!ok) return SKEW_CUDA_ERROR;
@@ -1264,6 +1266,7 @@ static int eigen_run(skew_batch_plan_t P, const double* const* A, double* const*
     // leave most of the GPU idle at the end
     E.back_off = P->e_back_off;
     E.back_items = P->back_items;
+    E.back_large = P->back_large;
     const int bgrid = (int)std::max<int64_t>(1, std::min<int64_t>(2 * (int64_t)P->h->sms, P->back_items));
     CK(launch_eigen_back(E, bgrid, P->nmax, st));
   }

@@ -15,6 +15,7 @@
 // are below 2 (1023) throughout; a column that comes larger takes 2^12 more, one that is
 // not finite stays NaN.  VT and T are measured.
 #pragma once
+#include <algorithm>
 #include <atomic>
 
 #include "skew_common.cuh"
@@ -28,6 +29,8 @@ struct BK {
   static constexpr int PB = CX ? 64 : 128;  // reflectors per panel: 128 rows of W fill a tile
   static constexpr int R = CX ? 2 : 1;      // doubles per entry
 };
+
+constexpr int BACK_SLICE = 65535;  // matrices per launch: the largest grid in y and z
 
 // One matrix.  nref reflectors: column c of A below the diagonal, v[c + 1] = 1, zero above.
 template <bool CX>
@@ -247,10 +250,11 @@ struct BackX {
 };
 
 // Src: bool get(int b, BackTask<CX>&) const: matrix b, false if there is nothing to do.
+// A launch takes the matrices b0, b0 + 1, ...: as many as a grid's y or z may count.
 template <bool CX, class Src>
-__global__ void __launch_bounds__(256) back_ex_kernel(Src S) {  // grid (columns / 8, count)
+__global__ void __launch_bounds__(256) back_ex_kernel(Src S, int b0) {  // grid (columns / 8, count)
   BackTask<CX> B;
-  if (!S.get(blockIdx.y, B)) return;
+  if (!S.get(b0 + blockIdx.y, B)) return;
   const int j = blockIdx.x * 8 + (threadIdx.x >> 5);
   if (j >= B.cols()) return;
   const double* x = B.column(j);
@@ -261,10 +265,10 @@ __global__ void __launch_bounds__(256) back_ex_kernel(Src S) {  // grid (columns
 }
 
 template <bool CX, class Src>
-__global__ void __launch_bounds__(OZ_NT, 1) back_gram_kernel(Src S) {  // grid (column tiles, panels, count)
+__global__ void __launch_bounds__(OZ_NT, 1) back_gram_kernel(Src S, int b0) {  // grid (column tiles, panels, count)
   extern __shared__ __align__(1024) unsigned char oz_buf[];
   BackGram<CX> P;
-  if (!S.get(blockIdx.z, P.B)) return;
+  if (!S.get(b0 + blockIdx.z, P.B)) return;
   P.p = blockIdx.y;
   const int c0 = P.p * BK<CX>::PB, nb = min(BK<CX>::PB, P.B.nref - c0);
   if ((int)blockIdx.x * OZ_N >= nb) return;
@@ -275,11 +279,11 @@ __global__ void __launch_bounds__(OZ_NT, 1) back_gram_kernel(Src S) {  // grid (
 // T(i, i) = tau_i, T(0:i, i) = -tau_i T(0:i, 0:i) G(0:i, i), in place of G: one CTA per
 // panel, grid (panels, count).  Thread j + PB q takes every fourth (eighth) term of row j.
 template <bool CX, class Src>
-__global__ void __launch_bounds__(512) back_tfac_kernel(Src S) {
+__global__ void __launch_bounds__(512) back_tfac_kernel(Src S, int b0) {
   constexpr int PB = BK<CX>::PB, R = BK<CX>::R, Q = 512 / PB;
   extern __shared__ __align__(16) double tf[];  // T (PB x (PB + 1) entries), partial sums (512 entries)
   BackTask<CX> B;
-  if (!S.get(blockIdx.y, B)) return;
+  if (!S.get(b0 + blockIdx.y, B)) return;
   const int c0 = blockIdx.x * PB, nb = min(PB, B.nref - c0);
   if (nb <= 0) return;
   const int ldt = B.ldt(), j = threadIdx.x % PB, q = threadIdx.x / PB;
@@ -337,10 +341,10 @@ __global__ void __launch_bounds__(512) back_tfac_kernel(Src S) {
 }
 
 template <bool CX, class Src>
-__global__ void __launch_bounds__(OZ_NT, 1) back_vt_kernel(Src S, int rt) {  // grid (row tiles x column tiles, panels, count)
+__global__ void __launch_bounds__(OZ_NT, 1) back_vt_kernel(Src S, int b0, int rt) {  // grid (row tiles x column tiles, panels, count)
   extern __shared__ __align__(1024) unsigned char oz_buf[];
   BackVT<CX> P;
-  if (!S.get(blockIdx.z, P.B)) return;
+  if (!S.get(b0 + blockIdx.z, P.B)) return;
   P.p = blockIdx.y;
   const int c0 = P.p * BK<CX>::PB, nb = min(BK<CX>::PB, P.B.nref - c0);
   const int i0 = (int)(blockIdx.x % rt) * OZ_M, j0 = (int)(blockIdx.x / rt) * OZ_N;
@@ -350,10 +354,10 @@ __global__ void __launch_bounds__(OZ_NT, 1) back_vt_kernel(Src S, int rt) {  // 
 }
 
 template <bool CX, class Src>
-__global__ void __launch_bounds__(256) back_evt_kernel(Src S) {  // grid (rows / 256, panels, count)
+__global__ void __launch_bounds__(256) back_evt_kernel(Src S, int b0) {  // grid (rows / 256, panels, count)
   constexpr int R = BK<CX>::R;
   BackTask<CX> B;
-  if (!S.get(blockIdx.z, B)) return;
+  if (!S.get(b0 + blockIdx.z, B)) return;
   const int p = blockIdx.y, c0 = p * BK<CX>::PB, nb = min(BK<CX>::PB, B.nref - c0);
   const int i = blockIdx.x * 256 + threadIdx.x;  // row of the real matrix
   if (nb <= 0 || i >= R * (B.n - c0 - 1)) return;
@@ -367,10 +371,10 @@ __global__ void __launch_bounds__(256) back_evt_kernel(Src S) {  // grid (rows /
 
 // step: panels from the last one, each matrix its own; grid (column tiles, splits, count)
 template <bool CX, class Src>
-__global__ void __launch_bounds__(OZ_NT, 1) back_w_kernel(Src S, int step) {
+__global__ void __launch_bounds__(OZ_NT, 1) back_w_kernel(Src S, int b0, int step) {
   extern __shared__ __align__(1024) unsigned char oz_buf[];
   BackW<CX> P;
-  if (!S.get(blockIdx.z, P.B)) return;
+  if (!S.get(b0 + blockIdx.z, P.B)) return;
   const int p = P.B.panels() - 1 - step;
   if (p < 0 || (int)blockIdx.x * OZ_N >= P.B.cols()) return;
   const int c0 = p * BK<CX>::PB, nb = min(BK<CX>::PB, P.B.nref - c0);
@@ -385,9 +389,9 @@ __global__ void __launch_bounds__(OZ_NT, 1) back_w_kernel(Src S, int step) {
 }
 
 template <bool CX, class Src>
-__global__ void back_join_kernel(Src S, int splits) {  // the splits' sums of W; grid (chunks, count)
+__global__ void back_join_kernel(Src S, int b0, int splits) {  // the splits' sums of W; grid (chunks, count)
   BackTask<CX> B;
-  if (!S.get(blockIdx.y, B)) return;
+  if (!S.get(b0 + blockIdx.y, B)) return;
   const size_t len = BK<CX>::R * (size_t)B.ldt() * B.cols();
   for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < len; q += (size_t)gridDim.x * blockDim.x) {
     double s = B.w[len + q];
@@ -397,10 +401,10 @@ __global__ void back_join_kernel(Src S, int splits) {  // the splits' sums of W;
 }
 
 template <bool CX, class Src>
-__global__ void __launch_bounds__(OZ_NT, 1) back_x_kernel(Src S, int step, int rt) {  // grid (row x column tiles, count)
+__global__ void __launch_bounds__(OZ_NT, 1) back_x_kernel(Src S, int b0, int step, int rt) {  // grid (row x column tiles, count)
   extern __shared__ __align__(1024) unsigned char oz_buf[];
   BackX<CX> P;
-  if (!S.get(blockIdx.y, P.B)) return;
+  if (!S.get(b0 + blockIdx.y, P.B)) return;
   P.p = P.B.panels() - 1 - step;
   if (P.p < 0) return;
   P.c0 = P.p * BK<CX>::PB;
@@ -439,17 +443,20 @@ inline cudaError_t back_transform_oz(const Src& S, int count, int nmax, int nref
     return e;
   const int ct = (cols_max + OZ_N - 1) / OZ_N, rt = (R * nmax + OZ_M - 1) / OZ_M, pt = PB / OZ_N;
   const size_t tf = sizeof(double) * R * (PB * (PB + 1) + 512);
-  back_ex_kernel<CX, Src><<<dim3((cols_max + 7) / 8, count), 256, 0, st>>>(S);
-  back_gram_kernel<CX, Src><<<dim3(pt, np, count), OZ_NT, OZ_SMEM, st>>>(S);
-  back_tfac_kernel<CX, Src><<<dim3(np, count), 512, tf, st>>>(S);
-  back_vt_kernel<CX, Src><<<dim3(rt * pt, np, count), OZ_NT, OZ_SMEM, st>>>(S, rt);
-  back_evt_kernel<CX, Src><<<dim3((R * nmax + 255) / 256, np, count), 256, 0, st>>>(S);
-  if ((e = cudaGetLastError())) return e;
-  for (int q = 0; q < np; q++) {
-    back_w_kernel<CX, Src><<<dim3(ct, splits, count), OZ_NT, OZ_SMEM, st>>>(S, q);
-    if (splits > 1) back_join_kernel<CX, Src><<<dim3(64, count), 256, 0, st>>>(S, splits);
-    back_x_kernel<CX, Src><<<dim3(rt * ct, count), OZ_NT, OZ_SMEM, st>>>(S, q, rt);
+  for (int b0 = 0; b0 < count; b0 += BACK_SLICE) {
+    const int m = std::min(count - b0, BACK_SLICE);
+    back_ex_kernel<CX, Src><<<dim3((cols_max + 7) / 8, m), 256, 0, st>>>(S, b0);
+    back_gram_kernel<CX, Src><<<dim3(pt, np, m), OZ_NT, OZ_SMEM, st>>>(S, b0);
+    back_tfac_kernel<CX, Src><<<dim3(np, m), 512, tf, st>>>(S, b0);
+    back_vt_kernel<CX, Src><<<dim3(rt * pt, np, m), OZ_NT, OZ_SMEM, st>>>(S, b0, rt);
+    back_evt_kernel<CX, Src><<<dim3((R * nmax + 255) / 256, np, m), 256, 0, st>>>(S, b0);
     if ((e = cudaGetLastError())) return e;
+    for (int q = 0; q < np; q++) {
+      back_w_kernel<CX, Src><<<dim3(ct, splits, m), OZ_NT, OZ_SMEM, st>>>(S, b0, q);
+      if (splits > 1) back_join_kernel<CX, Src><<<dim3(64, m), 256, 0, st>>>(S, b0, splits);
+      back_x_kernel<CX, Src><<<dim3(rt * ct, m), OZ_NT, OZ_SMEM, st>>>(S, b0, q, rt);
+      if ((e = cudaGetLastError())) return e;
+    }
   }
   return cudaSuccess;
 }

@@ -914,8 +914,8 @@ size_t eigen_work_doubles(int n) {
 
 struct BatchBack {
   EigenBatch E;
-  __device__ bool get(int b, BackTask<false>& T) const {
-    const int n = E.n[b];
+  __device__ bool get(int t, BackTask<false>& T) const {
+    const int b = E.order[t], n = E.n[b];
     if (n < kBackOzMin || E.status[b] == SKEW_NO_CONVERGENCE) return false;
     const bool qonly = E.back_q && E.fsel && E.fsel[b] == 1;
     T.A = E.refl[b];
@@ -972,7 +972,8 @@ cudaError_t launch_eigen_vectors(const EigenBatch& E, int grid, cudaStream_t st)
 }
 
 // Matrices below kBackOzMin: reflector blocks of 8 on the FP64 pipe, items of column
-// chunks; from it on, panels on the tensor cores (skew_back.cuh), all matrices at a time.
+// chunks; from it on (the first E.back_large in the processing order), panels on the tensor
+// cores (skew_back.cuh), all of them at a time.
 cudaError_t launch_eigen_back(const EigenBatch& E, int grid, int nmax, cudaStream_t st) {
   cudaError_t e;
   if (E.back_items > 0) {
@@ -982,9 +983,9 @@ cudaError_t launch_eigen_back(const EigenBatch& E, int grid, int nmax, cudaStrea
     eigen_back_kernel<<<grid, ENT, smem, st>>>(E);
     if ((e = cudaGetLastError())) return e;
   }
-  if (nmax < kBackOzMin) return cudaSuccess;
+  if (E.back_large == 0) return cudaSuccess;
   BatchBack S{E};
-  return back_transform_oz<false>(S, E.count, nmax, nmax - 2, 2 * nmax, 1, st);
+  return back_transform_oz<false>(S, E.back_large, nmax, nmax - 2, 2 * nmax, 1, st);
 }
 
 // ---------------------------------------------------------------------------

@@ -261,6 +261,7 @@ struct EigenBatch {
   const int32_t* back_off = nullptr;  // [count + 1] back-transformation items before each matrix
                              // of the processing order (null: one item per matrix)
   int32_t back_items = 0;    // total items (chunks of kBackCols columns)
+  int32_t back_large = 0;    // matrices from kBackOzMin on
   int back_q = 0;            // 1: the real Schur basis Q was built in the tridiagonal basis
                              // (pwork block 0): the back-transformation takes Q alone for the
                              // matrices with fsel = 1, and the adjoint starts from it

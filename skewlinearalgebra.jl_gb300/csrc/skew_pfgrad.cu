@@ -165,13 +165,18 @@ cudaError_t launch_pfgrad(const PfGrad& P, int count, int nmax, cudaStream_t st)
   static std::atomic<uint64_t> raised{0};
   cudaError_t e = raise_smem_limit_once((const void*)pg_product_kernel, raised);
   if (e != cudaSuccess) return e;
-  pg_identity_kernel<<<dim3(std::max(1, nmax * nmax / 2048), count), 256, 0, st>>>(P);
-  PgBack S{P};
-  if ((e = back_transform_oz<false>(S, count, nmax, nmax - 2, nmax, 1, st))) return e;
-  pg_solve_kernel<<<dim3((nmax + 127) / 128, count), 128, sizeof(double) * nmax, st>>>(P);
   const int tiles = ((nmax + OZ_M - 1) / OZ_M) * ((nmax + OZ_N - 1) / OZ_N);
-  pg_product_kernel<<<dim3(tiles, count), OZ_NT, OZ_SMEM, st>>>(P);
-  return cudaGetLastError();
+  for (int b0 = 0; b0 < count; b0 += BACK_SLICE) {
+    const int m = std::min(count - b0, BACK_SLICE);
+    PfGrad Q = P;
+    Q.order += b0;
+    pg_identity_kernel<<<dim3(std::max(1, nmax * nmax / 2048), m), 256, 0, st>>>(Q);
+    if ((e = back_transform_oz<false>(PgBack{Q}, m, nmax, nmax - 2, nmax, 1, st))) return e;
+    pg_solve_kernel<<<dim3((nmax + 127) / 128, m), 128, sizeof(double) * nmax, st>>>(Q);
+    pg_product_kernel<<<dim3(tiles, m), OZ_NT, OZ_SMEM, st>>>(Q);
+    if ((e = cudaGetLastError())) return e;
+  }
+  return cudaSuccess;
 }
 
 }  // namespace skew
