@@ -1020,6 +1020,10 @@ __global__ void set8_kernel(double** dst, double* a, double* b, double* c, doubl
   dst[7] = h;
 }
 __global__ void copy_status_kernel(const int* src, int* dst) { *dst = *src; }
+__global__ void set_size_kernel(int32_t* n, int32_t value, int* status) {
+  *n = value;
+  *status = SKEW_OK;
+}
 }  // namespace
 
 static int eigen_ws(skew_batch_plan_t P) {
@@ -1457,9 +1461,9 @@ static int func_large(skew_handle_t h, double* A, const double* ev, int64_t n, d
   int32_t* dn = (int32_t*)(ptrs + 8);
   int* status = (int*)(dn + 1);
   int* exps = (int*)(ptrs + 8 + 2);
-  const int32_t n32 = (int32_t)n;
-  CK(cudaMemcpyAsync(dn, &n32, sizeof(int32_t), cudaMemcpyHostToDevice, s));  // pageable: staged before return
-  CK(cudaMemsetAsync(status, 0, sizeof(int), s));
+  // by a kernel: a captured copy would read this stack again at every replay
+  set_size_kernel<<<1, 1, 0, s>>>(dn, (int32_t)n, status);
+  CK(cudaGetLastError());
   if (A) {
     st = eigen_large(h, A, n, n, vals, Vr, Vi, n, status);
   } else {
