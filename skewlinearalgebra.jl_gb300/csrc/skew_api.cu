@@ -87,7 +87,7 @@ struct skew_batch_plan_st {
   // gradients of log|Pf| on the tensor cores (global-memory buckets): allocated on first use
   double* pg_ws = nullptr;
   double* pg_tau = nullptr;
-  double** pg_refl = nullptr;  // [count] a matrix's workspace, null outside those buckets
+  double** pg_refl = nullptr;  // [count] a matrix's workspace, null outside those buckets and for odd n
   int pg_state = 0;            // 0: not tried, 1: ready, -1: no memory (the fused kernel runs)
   int* e_exps = nullptr;  // exponents of the tiled products' operands (2 x ev_total)
   int* e_fsel = nullptr;  // exp adjoint: per matrix, real Schur-basis (1) or complex (0) form
@@ -721,6 +721,7 @@ static int pfgrad_ws(skew_batch_plan_t P) {
   for (const Bucket& B : P->buckets) {
     if (B.smem_matrix) continue;
     for (int t = B.begin; t < B.end; t++) {
+      if (P->n_host[order[t]] & 1) continue;  // no Pfaffian, no gradient
       off[order[t]] = total;
       total += pfgrad_ws_doubles(P->n_host[order[t]]);
     }

@@ -866,8 +866,7 @@ __device__ void run_job(const Job& J, const MW& W, bool inplace, const Smem& s) 
     __syncthreads();
     return;
   }
-  const bool odd = (n & 1);
-  if (J.want_pf && odd) {  // pfaffian.jl:169
+  if (J.want_pf && (n & 1)) {  // pfaffian.jl:169
     if (threadIdx.x == 0) {
       *J.logpf = -INFINITY;
       *J.sign = 0.0;
@@ -875,7 +874,7 @@ __device__ void run_job(const Job& J, const MW& W, bool inplace, const Smem& s) 
     }
     if (J.G) fill<NT>(G, n, nan(""));
     __syncthreads();
-    if (!J.ev_out) return;
+    return;  // nothing to reduce, also where the tensor-core gradients ask for ev
   }
   forward<NT>(W, n, s);
   if (J.refl_out) {
@@ -890,8 +889,8 @@ __device__ void run_job(const Job& J, const MW& W, bool inplace, const Smem& s) 
       if (J.ev_out) J.ev_out[a] = s.ev[a];
       if (J.tau_out) J.tau_out[a] = s.tau[a];
     }
-  if (!J.want_pf || odd) {
-    if (threadIdx.x == 0 && J.status && !J.want_pf) *J.status = SKEW_OK;
+  if (!J.want_pf) {
+    if (threadIdx.x == 0 && J.status) *J.status = SKEW_OK;
     __syncthreads();
     return;
   }
