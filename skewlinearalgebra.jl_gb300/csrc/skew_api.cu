@@ -43,13 +43,14 @@ struct Bucket {
   int split = 0;     // > begin: the work median of the slice (two regions, see batch_kernel)
   int grid_wide = 0;  // > 0: CTAs of 16 warps, one per SM (functions of the matrices)
   size_t gws_off;    // offset of the bucket's slots in the plan workspace (doubles)
+  int pg_begin = 0, pg_end = 0, pg_nmax = 0;  // gradients on the tensor cores: slice of the plan's pg_order
 };
 
 struct skew_batch_plan_st {
   skew_handle_t h = nullptr;
   Tuning tune;  // the handle's table when the plan was created (bucket shapes)
   int64_t count = 0;
-  std::vector<int32_t> n_host;
+  std::vector<int32_t> n_host, order_host;  // sizes; processing order (largest first)
   std::vector<Bucket> buckets;
   int32_t* d_n = nullptr;
   int32_t* d_order = nullptr;
@@ -84,10 +85,11 @@ struct skew_batch_plan_st {
   double** e_p_work = nullptr;     // work + off_w per matrix
   int* e_status = nullptr;
   unsigned* e_counter = nullptr;
-  // gradients of log|Pf| on the tensor cores (global-memory buckets): allocated on first use
-  double* pg_ws = nullptr;
+  // gradients of log|Pf| on the tensor cores (see pg_takes): one allocation, on first use
+  double* pg_ws = nullptr;     // the matrices' workspaces | pg_tau | pg_refl | pg_order
   double* pg_tau = nullptr;
-  double** pg_refl = nullptr;  // [count] a matrix's workspace, null outside those buckets and for odd n
+  double** pg_refl = nullptr;  // [count] a matrix's workspace, null for the others
+  int32_t* pg_order = nullptr;  // the matrices, largest first
   int pg_state = 0;            // 0: not tried, 1: ready, -1: no memory (the fused kernel runs)
   int* e_exps = nullptr;  // exponents of the tiled products' operands (2 x ev_total)
   int* e_fsel = nullptr;  // exp adjoint: per matrix, real Schur-basis (1) or complex (0) form
@@ -550,6 +552,7 @@ int skew_batch_plan_create(skew_handle_t h, const int64_t* n, int64_t count, ske
   std::vector<int32_t> order(count);
   std::iota(order.begin(), order.end(), 0);
   std::stable_sort(order.begin(), order.end(), [&](int32_t a, int32_t b) { return P->n_host[a] > P->n_host[b]; });
+  P->order_host = order;
   std::vector<int64_t> ev_off(count);
   int64_t acc = 0;
   for (int64_t b = 0; b < count; b++) {
@@ -684,7 +687,7 @@ int skew_batch_plan_destroy(skew_batch_plan_t P) {
   void* eig[] = {P->e_refl, P->e_tau, P->e_evb, P->e_G, P->e_log, P->e_work, P->e_vr, P->e_vi, P->e_vals,
                  P->e_off_log, P->e_cap_log, P->e_log_len, P->e_off_w, P->e_p_refl, P->e_p_vr, P->e_p_vi,
                  P->e_p_vals, P->e_p_scratch, P->e_p_work, P->e_status, P->e_fsel, P->e_exps, P->e_back_off,
-                 P->e_counter, P->pg_ws, P->pg_tau, P->pg_refl};
+                 P->e_counter, P->pg_ws};
   for (void* q : eig)
     if (q) cudaFreeAsync(q, st);
   if (P->fv_idx) cudaFreeAsync(P->fv_idx, st);
@@ -701,8 +704,24 @@ int skew_batch_plan_destroy(skew_batch_plan_t P) {
   return SKEW_OK;
 }
 
-// Workspace of the tensor-core gradients.  Without the memory for it the plan keeps the
-// fused kernel, which needs none.
+// Whether the gradients of a bucket of `many` even matrices of sizes lo .. hi (working copies in
+// global memory) are formed on the tensor cores.  Beside the fused kernel, whole call, they are
+// faster at n = 108 .. 128 and from 138 on (300 and 1500 matrices of n = 108 0.97 and 0.96,
+// 128 0.89 and 0.88, 140 1.02 and 1.00, 148 0.97 and 0.95, 160 0.93 and 0.89, 256 0.72, 258
+// 0.80).  At the other sizes the padding of the 128-row tiles and panels costs as much as they
+// save, and it depends on how full the fused kernel's rounds of two CTAs per SM are: up to one
+// and a half matrices per SM, 64 of n = 98 0.82, 152 0.94, 228 0.96, 240 1.03, 304 1.05, 400
+// 0.91, 608 1.04, 620 0.96, 700 1.03, 1216 1.05, 2500 1.06; of n = 130 64 0.86, 228 1.00, 304
+// 1.09, 400 0.90, 608 1.08, 620 0.99, 700 1.07, 2500 1.08.  Mixed sizes stay together: 4096 of
+// n = 16 .. 256 57.7 ms, with the ones that fit badly in the fused kernel 58.2.
+static bool pg_takes(int lo, int hi, int64_t many, int sms) {
+  if (hi >= 108 && (lo <= 128 || hi > 136)) return true;
+  const int64_t round = 2 * (int64_t)sms, rounds = (many + round - 1) / round;
+  return 4 * many <= 3 * round || 100 * many < 76 * rounds * round;
+}
+
+// Workspace of the tensor-core gradients, about 4.6 n^2 doubles per matrix.  Without the memory
+// for it the plan keeps the fused kernel, which needs none.
 static int pfgrad_ws(skew_batch_plan_t P) {
   if (P->pg_state != 0) return SKEW_OK;
   cudaStream_t st = P->h->stream;
@@ -713,39 +732,47 @@ static int pfgrad_ws(skew_batch_plan_t P) {
     return SKEW_OK;
   }
   P->pg_state = -1;
-  std::vector<int32_t> order(P->count);
-  std::iota(order.begin(), order.end(), 0);
-  std::stable_sort(order.begin(), order.end(), [&](int32_t a, int32_t c) { return P->n_host[a] > P->n_host[c]; });
-  std::vector<size_t> off(P->count, SIZE_MAX);
+  std::vector<int32_t> list;
+  std::vector<size_t> off;
   size_t total = 0;
-  for (const Bucket& B : P->buckets) {
+  for (Bucket& B : P->buckets) {
     if (B.smem_matrix) continue;
+    int lo = 0, hi = 0;
+    int64_t many = 0;
     for (int t = B.begin; t < B.end; t++) {
-      if (P->n_host[order[t]] & 1) continue;  // no Pfaffian, no gradient
-      off[order[t]] = total;
-      total += pfgrad_ws_doubles(P->n_host[order[t]]);
+      const int n = P->n_host[P->order_host[t]];
+      if (n & 1) continue;  // no Pfaffian, no gradient
+      lo = n;
+      hi = std::max(hi, n);
+      many++;
     }
+    if (many == 0 || !pg_takes(lo, hi, many, P->h->sms)) continue;
+    B.pg_begin = (int)list.size();
+    B.pg_nmax = hi;
+    for (int t = B.begin; t < B.end; t++) {
+      const int32_t b = P->order_host[t], n = P->n_host[b];
+      if (n & 1) continue;
+      list.push_back(b);
+      off.push_back(total);
+      total += pfgrad_ws_doubles(n);
+    }
+    B.pg_end = (int)list.size();
   }
-  if (total == 0) return SKEW_OK;
-  auto alloc = [&](auto** p, size_t bytes) {
-    if (cudaMallocAsync(p, bytes, st) == cudaSuccess) return true;
+  if (list.empty()) return SKEW_OK;
+  const size_t tail = (size_t)P->ev_total + (size_t)P->count + (list.size() + 1) / 2;
+  if (cudaMallocAsync(&P->pg_ws, sizeof(double) * (total + tail), st) != cudaSuccess) {
     (void)cudaGetLastError();
-    *p = nullptr;
-    return false;
-  };
-  if (!alloc(&P->pg_ws, sizeof(double) * total) || !alloc(&P->pg_tau, sizeof(double) * P->ev_total) ||
-      !alloc(&P->pg_refl, sizeof(double*) * P->count)) {
-    if (P->pg_ws) CK(cudaFreeAsync(P->pg_ws, st));
-    if (P->pg_tau) CK(cudaFreeAsync(P->pg_tau, st));
     P->pg_ws = nullptr;
-    P->pg_tau = nullptr;
     return SKEW_OK;
   }
+  P->pg_tau = P->pg_ws + total;
+  P->pg_refl = (double**)(P->pg_tau + P->ev_total);
+  P->pg_order = (int32_t*)(P->pg_refl + P->count);
   std::vector<double*> ptr(P->count, nullptr);
-  for (int64_t b = 0; b < P->count; b++)
-    if (off[b] != SIZE_MAX) ptr[b] = P->pg_ws + off[b];
+  for (size_t k = 0; k < list.size(); k++) ptr[list[k]] = P->pg_ws + off[k];
   CK(cudaMemcpyAsync(P->pg_refl, ptr.data(), sizeof(double*) * P->count, cudaMemcpyHostToDevice, st));
-  CK(cudaStreamSynchronize(st));  // ptr goes out of scope
+  CK(cudaMemcpyAsync(P->pg_order, list.data(), sizeof(int32_t) * list.size(), cudaMemcpyHostToDevice, st));
+  CK(cudaStreamSynchronize(st));  // the host vectors go out of scope
   P->pg_state = 1;
   return SKEW_OK;
 }
@@ -788,19 +815,19 @@ static int run_buckets(skew_batch_plan_t P, const double* const* A, double* logp
       bp.split = B.begin;
     }
     bp.grad_host = grad_host;
-    // gradients of the global-memory matrices: the reduction alone, then the products of all
-    // of them on the tensor cores
-    const bool pg = grad && !B.smem_matrix && !host_in && !grad_host && P->pg_state == 1;
+    // gradients on the tensor cores: the reduction alone (a matrix without pg_refl forms its
+    // gradient there), then the products of all of them
+    const bool pg = grad && !host_in && !grad_host && P->pg_state == 1 && B.pg_end > B.pg_begin;
     if (pg) {
-      bp.grad = nullptr;
       bp.ev_out = P->d_ev;
       bp.tau_out = P->pg_tau;
       bp.refl_out = P->pg_refl;
+      bp.refl_grad = 1;
     }
     CK(launch_batch_pf(bp, grid, st, tridiag_only));
     if (pg) {
       PfGrad g;
-      g.order = P->d_order + B.begin;
+      g.order = P->pg_order + B.pg_begin;
       g.n = P->d_n;
       g.off = P->d_ev_off;
       g.ev = P->d_ev;
@@ -808,7 +835,7 @@ static int run_buckets(skew_batch_plan_t P, const double* const* A, double* logp
       g.refl = P->pg_refl;
       g.grad = grad;
       g.status = status;
-      CK(launch_pfgrad(g, B.end - B.begin, B.nmax, st));
+      CK(launch_pfgrad(g, B.pg_end - B.pg_begin, B.pg_nmax, st));
     }
   }
   return SKEW_OK;

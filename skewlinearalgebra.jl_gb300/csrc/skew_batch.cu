@@ -969,6 +969,7 @@ __global__ void __launch_bounds__(NT) batch_kernel(BatchParams P, int tridiag_on
     J.ev_out = P.ev_out ? P.ev_out + P.ev_off[b] : nullptr;
     J.tau_out = P.tau_out ? P.tau_out + P.ev_off[b] : nullptr;
     J.refl_out = P.refl_out ? P.refl_out[b] : nullptr;
+    if (P.refl_grad && J.refl_out) J.G = nullptr;
     J.status = tridiag_only ? nullptr : P.status + b;
     J.check = P.check != 0;
     J.want_pf = !tridiag_only;

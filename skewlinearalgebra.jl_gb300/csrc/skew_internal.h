@@ -96,6 +96,7 @@ struct BatchParams {
   const int64_t* ev_off;   // offsets into ev_out (and tau_out)
   double* tau_out;         // packed tau, same offsets, or null
   double* const* refl_out; // [count] n x n buffers receiving the reduced matrix (reflectors) or null
+  int32_t refl_grad = 0;   // matrices with a refl_out buffer leave their gradient to launch_pfgrad
   int* status;             // [count] or null
   int32_t nt = 0;          // threads per CTA (0: the default for the copy's location)
   int32_t host_in = 0;     // A[] point into page-locked host memory (read with more loads in flight)

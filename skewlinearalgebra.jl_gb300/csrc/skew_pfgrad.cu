@@ -142,7 +142,7 @@ struct PgTile {
   __device__ void timeout() const { *status = SKEW_TIMEOUT; }
 };
 
-// G = Y Q^T; a matrix without a gradient (odd, or a zero Pfaffian) gets NaN.  grid (tiles, count)
+// G = Y Q^T; a matrix without a gradient (a zero Pfaffian) gets NaN.  grid (tiles, count)
 __global__ void __launch_bounds__(OZ_NT, 1) pg_product_kernel(PfGrad P) {
   extern __shared__ __align__(1024) unsigned char oz_buf[];
   PgItem I;
