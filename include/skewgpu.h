@@ -72,6 +72,15 @@ SKEW_API int skew_set_stream(skew_handle_t handle, skew_stream_t stream);
 SKEW_API const char* skew_status_string(int status);
 SKEW_API int skew_version(void);
 
+/* Accuracy of the tensor-core paths (products of the matrix functions and adjoints, gradients and
+ * back-transformations above small sizes, reductions of one real matrix above n = 640 and of one
+ * complex matrix from n = 384).  Operands are held in 56 bits relative to the largest entry of a
+ * row, column or 64 x 64 tile, sums in 64 bits or more.  Errors are at most those of Float64
+ * arithmetic relative to these largest entries: backward stable norm-wise.  An entry that is much
+ * smaller than its neighbours keeps fewer bits than in an entry-by-entry Float64 product, so the
+ * small blocks of graded operands (a cotangent D C D with D over many orders of magnitude) come
+ * with errors relative to the large ones they share a row or column with. */
+
 /* ---------------------------------------------------------------------------
  * Single-matrix entry points (real Float64).
  * ------------------------------------------------------------------------- */
@@ -141,8 +150,8 @@ SKEW_API int skew_eigen_d(skew_handle_t h, double* A, int64_t n, int64_t lda, do
                  int64_t ldv, int* info);
 
 /* Base.exp(A::SkewHermitian{Float64})  exp.jl:3-35, :48.  E (n x n) = exp(A). A destroyed.
- * Requires lda == lde == n.  Above n = 1024 the eigenpairs come from the large-matrix path
- * of skew_eigen_d (their order does not change the function). */
+ * Requires lda == lde == n.  From n = 96 on the eigenpairs come from the large-matrix path
+ * of skew_eigen_d, on the whole GPU (their order does not change the function). */
 SKEW_API int skew_exp_d(skew_handle_t h, double* A, int64_t n, int64_t lda, double* E, int64_t lde, int* info);
 
 /* Base.cis(A::SkewHermitian{Float64})  exp.jl:99-110, :204.  C = cis(A) = exp(iA), Hermitian,
@@ -159,7 +168,11 @@ SKEW_API int skew_batch_plan_destroy(skew_batch_plan_t plan);
 
 /* logabspfaffian for every matrix; A[b] (device array of device pointers) is read only,
  * leading dimension n[b].  grad may be NULL; otherwise grad[b] receives 1/2 A_b^{-T}
- * (leading dimension n[b]).  status[b] is a skew_status_t per matrix. */
+ * (leading dimension n[b]).  status[b] is a skew_status_t per matrix.
+ * The first call with grad (outside a capture) allocates about 4.6 n^2 doubles for every even
+ * matrix above n = 96 whose gradient is formed on the tensor cores, and waits for the stream; the
+ * plan keeps them until it is destroyed.  Without that memory the gradients are formed one CTA
+ * per matrix, in no workspace. */
 SKEW_API int skew_batch_logabspf_d(skew_batch_plan_t plan, const double* const* A, double* logpf, double* sign,
                           double* const* grad, int* status);
 
@@ -184,7 +197,9 @@ SKEW_API int skew_batch_eigvals_d(skew_batch_plan_t plan, const double* const* A
 SKEW_API int skew_batch_eigen_d(skew_batch_plan_t plan, const double* const* A, double* const* vals_im,
                                 double* const* Vr, double* const* Vi, int* status);
 
-/* exp(A_b) for every matrix (skewexp!, exp.jl:3-35): E[b] n x n real, leading dimension n. */
+/* exp(A_b) for every matrix (skewexp!, exp.jl:3-35): E[b] n x n real, leading dimension n.
+ * The plan's first function call allocates eigenvector workspace for up to four size groups at a
+ * time, at most 256 MB each (one matrix, if that needs more). */
 SKEW_API int skew_batch_exp_d(skew_batch_plan_t plan, const double* const* A, double* const* E, int* status);
 
 /* cis(A_b) = exp(i A_b) for every matrix (skewcis!, exp.jl:99-110): C[b] n x n ComplexF64

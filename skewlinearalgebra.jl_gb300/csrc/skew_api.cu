@@ -1440,7 +1440,7 @@ static int single_func(skew_handle_t h, double* A, int64_t n, int64_t lda, doubl
   return SKEW_OK;
 }
 
-// Large single matrices (n > 1024): blocked reduction, bisection and the
+// One matrix on the whole GPU (eigen above n = 1024, functions from n = 96): reduction, bisection and the
 // twisted-factorisation eigenvectors of skew_tdvec.cu (the reference's fallback
 // formulation, values sorted descending).
 static int eigen_large(skew_handle_t h, double* A, int64_t n, int64_t lda, double* vals_im, double* Vr, double* Vi,
@@ -1467,8 +1467,8 @@ static int eigen_large(skew_handle_t h, double* A, int64_t n, int64_t lda, doubl
   return SKEW_OK;
 }
 
-// exp, cis, the other matrix functions and the exp adjoint of one large matrix
-// (n > 1024): the eigenpairs come from eigen_large (dense A, destroyed) or from
+// exp, cis, the other matrix functions and the exp adjoint of one matrix (dense A from
+// n = 96, tridiagonal ev above 1024): the eigenpairs come from eigen_large (dense A, destroyed) or from
 // bisection and twisted vectors of the tridiagonal ev; then the element-wise step
 // and the tiled products of the batched path run on them as a batch of one.  The
 // eigenvalue order (descending here) does not change these functions.
@@ -1591,10 +1591,10 @@ static int zlayout(skew_handle_t h, int64_t n, int64_t B, bool copy, bool vecs, 
   return SKEW_OK;
 }
 
-// complex reduction in place.  One matrix: one CTA for n <= 128, the persistent
+// complex reduction in place.  One matrix: one cluster of CTAs for n <= 128, the persistent
 // blocked kernel from the tuning key zpersist_min_n, per-column multi-CTA
 // kernels between (and where the persistent kernel cannot run).  B > 1 matrices of
-// size n, n^2 apart: one CTA each.
+// size n, n^2 apart: a cluster of 1 to 8 CTAs each.
 static int64_t zpersist_min_n(skew_handle_t h) { return h->tune.zpersist_min_n; }
 
 static int zreduce(skew_handle_t h, double* A, int64_t n, int64_t lda, int64_t B, double* tau, double* ev,

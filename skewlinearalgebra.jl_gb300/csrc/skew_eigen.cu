@@ -1,5 +1,6 @@
 // Eigenvectors, exp, cis and the exp adjoint for real skew matrices (n <= 1024),
-// batched; single matrices run as a batch of one.
+// batched; a single matrix runs as a batch of one (functions below n = 96; from there on the
+// products alone, on eigenpairs of skew_tdvec.cu).
 //
 // Pipeline (after the batched reduction of skew_batch.cu has left the
 // reflectors, tau and ev of every matrix in the plan's workspace):
@@ -869,9 +870,6 @@ static cudaError_t bgemm(const EigenBatch& E, int nterms, BOperand A0, BOperand 
   P.c_add_sq = c_add_sq;
   P.c_add = c_add;
   P.c_step = c_step;
-  P.off_n = E.off_n;
-  P.exps = E.exps;
-  P.exps_stride = E.exps_stride;
   P.off_n = E.off_n;
   P.exps = E.exps;
   P.exps_stride = E.exps_stride;

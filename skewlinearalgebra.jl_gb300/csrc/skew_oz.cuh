@@ -14,7 +14,10 @@
 // entries the eight sums are joined in a 96-bit integer (2^-64 of the largest product),
 // whatever the length of the sum.  Measured against products summed in 113 bits (entries
 // N(0, 1), K = 16, 128, 512, 2048): 4.9e-17 to 5.2e-17 of the result, the rounding of the
-// result itself; FMAs 1.4e-16, 3.8e-16, 7.5e-16, 1.5e-15.  A vector with an infinity or a
+// result itself; FMAs 1.4e-16, 3.8e-16, 7.5e-16, 1.5e-15.  That is relative to the largest
+// entries: one below 1/8 of its vector's largest keeps fewer than 53 bits, so where large
+// entries meet zeros, a small result beside them is less accurate than by FMAs (block-diagonal
+// times a cotangent graded by 1e-6: its small block to 1.9e-11 instead of 2.4e-16).  A vector with an infinity or a
 // NaN (e = 2047) makes its results NaN.
 //
 // One CTA of 17 warps computes a 128 x 64 tile; its eight groups fill the SM's 512

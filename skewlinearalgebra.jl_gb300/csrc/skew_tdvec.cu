@@ -1,4 +1,5 @@
-// Eigenvectors of one large real skew matrix (n > 1024) on the whole GPU.
+// Eigenvectors of one real skew matrix on the whole GPU (eigen above n = 1024, functions
+// from n = 96).
 //
 // The reference solves the tridiagonal eigenproblem by implicit QR with the
 // rotations accumulated into Qodd / Qeven (skewtrieigen_divided!, skeweigen.jl:
