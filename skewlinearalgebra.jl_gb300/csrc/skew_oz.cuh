@@ -119,8 +119,8 @@ __device__ __forceinline__ void oz_mma(uint32_t d, uint64_t a, uint64_t b, uint3
       : "memory");
 }
 
-// Bounded wait for a phase of an mbarrier, by a whole warp (the lanes agree on the outcome:
-// warp-wide instructions follow).
+// Bounded wait for a phase of an mbarrier.  A lane may give up where its neighbours did not:
+// they vote before the next warp-wide instruction.
 __device__ __forceinline__ bool oz_wait(uint32_t bar, uint32_t parity) {
   for (int t = 0; t < OZ_POLLS; t++) {
     uint32_t done;
@@ -129,7 +129,7 @@ __device__ __forceinline__ bool oz_wait(uint32_t bar, uint32_t parity) {
         : "=r"(done)
         : "r"(bar), "r"(parity)
         : "memory");
-    if (__all_sync(0xffffffffu, done)) return true;
+    if (done) return true;
   }
   return false;
 }
@@ -297,7 +297,7 @@ __device__ __forceinline__ void oz_tile(const Prob& P, int i0, int j0, unsigned 
       }
       if (s + 1 < steps) fetch(s + 1);
       if (fresh && s > 0) {  // the previous sum is complete: join it before its accumulators start over
-        ok = ok && oz_wait(oz_smem(bars + (w ^ 1)), (uses[w ^ 1] - 1) & 1);
+        ok = __all_sync(0xffffffffu, ok && oz_wait(oz_smem(bars + (w ^ 1)), (uses[w ^ 1] - 1) & 1));
         if (ok) drain();
       }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -318,7 +318,7 @@ __device__ __forceinline__ void oz_tile(const Prob& P, int i0, int j0, unsigned 
   }
   if (ok && steps > 0 && worker) {
     const int w = (steps - 1) & 1;
-    ok = oz_wait(oz_smem(bars + w), (uses[w] - 1) & 1);
+    ok = __all_sync(0xffffffffu, oz_wait(oz_smem(bars + w), (uses[w] - 1) & 1));
     if (ok) drain();
   }
   if (!__syncthreads_and(ok)) {  // a wait gave up: what was issued ends before its memory is given back

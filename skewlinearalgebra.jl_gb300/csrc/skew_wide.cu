@@ -330,10 +330,7 @@ __device__ __forceinline__ bool fxp_matvec(const FxpPanel& P, FxpStream& S, int 
 #pragma unroll
     for (int qd = 0; qd < 4; qd++, q++) {
       const unsigned at = first + q;
-      if (!oz_wait(S.bar + 8 * (at % FXP_SLOTS), (at / FXP_SLOTS) & 1)) {
-        P.w.sync[1] = 1u;
-        return false;
-      }
+      const bool got = oz_wait(S.bar + 8 * (at % FXP_SLOTS), (at / FXP_SLOTS) & 1);
       const int4* src = reinterpret_cast<const int4*>(buf) + (at % FXP_SLOTS) * (FXP_TILE / 4 / 2) + lane;
       int cx[4], cy[4];
       long long ch[4], cm[4];
@@ -360,6 +357,7 @@ __device__ __forceinline__ bool fxp_matvec(const FxpPanel& P, FxpStream& S, int 
         }
       }
       __syncwarp();
+      if (!__all_sync(0xffffffffu, got)) return false;  // the whole warp, if one lane's wait gave up
       const bool want = q + FXP_SLOTS < S.quarters || more;  // the next column starts over
       if (want) {
         if (lane == 0) S.request((q + FXP_SLOTS) % S.quarters);
