@@ -423,6 +423,8 @@ def main():
     # the FP64 pipe, the other gradients' products on the tensor cores
     flops = float(flops_per_matrix(sizes).sum())
     achieved_tflops = flops / (ms_dev / args.steps / 1e3) / 1e12
+    n3 = np.asarray(sizes, dtype=np.float64) ** 3
+    on_fp64 = float((4.0 / 3.0 * n3).sum() + (2.0 * n3[np.asarray(sizes) <= skewgpu.tuning_get("batch_smem_nmax")]).sum())
 
     # plain per-matrix GPU path: single-matrix C-ABI call looped over a sample
     plain = None
@@ -542,7 +544,11 @@ def main():
                          "algorithmic_bytes_per_step": int(2 * total * 8),
                          "peak_source": "FP64 DFMA peak measured live by skew_measure_fp64_peak "
                                         "(MEASURED_PEAKS.json has no FP64 figure)",
-                         "algorithmic_flops_per_step": flops, "kernel": "batch_kernel"},
+                         "algorithmic_flops_per_step": flops, "kernel": "batch_kernel",
+                         "parts": {"fp64_pipe_flops": on_fp64, "tensor_core_flops": flops - on_fp64,
+                                   "fp64_pipe_frac_of_step": on_fp64 / (ms_dev / args.steps / 1e3) / 1e12 / fp64_peak,
+                                   "note": "reductions (and gradients up to n = 96) on the FP64 pipe, the other "
+                                           "gradients' products on the tensor cores, one after the other"}},
             "gpu_launches": int(args.steps * _launches_per_call(sizes)),
             "tuning": skewgpu.tuning_source(),
             "fp64_pipes_tflops": skewgpu.measure_fp64_pipes(),
